@@ -411,11 +411,12 @@ bilu_status bilu_probe_fp64_rate(double* h_gflops, double* h_sm_mhz, void* strea
  * (round to nearest even; the hardware conversion for float subnormal results,
  * infinities and NaNs) and the correctly rounded FP64 reciprocal of the FAST
  * ParILU and ISAI (against __drcp_rn; the hardware's for zero, subnormal,
- * infinite and NaN inputs and subnormal results), on n_per_thread bit patterns
- * per thread of 4 CTAs of 256 threads per SM: random doubles, doubles across
+ * infinite and NaN inputs and subnormal results) and the quotients formed from
+ * it (against the division), on n_per_thread bit patterns per thread of 4 CTAs of 256 threads per SM: random doubles, doubles across
  * every float exponent boundary with rounding ties, random floats, and
  * doubles with short, long and zero mantissas.  h_mismatch[0] / [1] / [2]:
- * roundings / widenings / reciprocals that differ (0, 0, 0 expected).
+ * roundings / widenings / reciprocals and quotients that differ (0, 0, 0
+ * expected).
  * Synchronises the stream.  No reference counterpart. */
 bilu_status bilu_check_integer_fp(int n_per_thread, uint64_t seed, unsigned long long* h_mismatch, void* stream);
 

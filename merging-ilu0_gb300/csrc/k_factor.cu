@@ -108,7 +108,10 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 
 // fast = true (BILU_REDUCE_FAST): the entries below the diagonal are
 // multiplied by reciprocals of the current diagonal, formed once per sweep,
-// instead of divided (n divisions per sweep instead of one per lower entry).
+// instead of divided; otherwise the quotient by u_jj is formed from the same
+// reciprocal (ifp::quot, the value of the division, in five FP64
+// instructions instead of ten or so).  recips: the n reciprocals fit beside
+// the two iterates (always, but for systems at the shared-memory limit).
 // TRACK: the ILU residual is formed (res_tol > 0 or res_out); a kernel of its
 // own, because FP64 instructions skipped under a runtime condition are
 // if-converted into predicated instructions that still take their FP64-unit
@@ -120,7 +123,7 @@ template <bool FAST, bool TRACK, bool SMALL>
 __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
     k_parilu0(const DevPattern P, int nsys, const double* __restrict__ A, const double* __restrict__ init,
               double* __restrict__ LUout, int sweeps, double res_tol, int* __restrict__ sweeps_out,
-              double* __restrict__ res_out) {
+              double* __restrict__ res_out, const int recips) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[32];
   const int sys = blockIdx.x;
@@ -130,7 +133,7 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
   // (instead of three arrays) fit two CTAs per SM at n = 1000
   double* cur = reinterpret_cast<double*>(smem);
   double* nxt = cur + nnz;
-  double* rinv = nxt + nnz;  // FAST only: n reciprocals
+  double* rinv = nxt + nnz;  // n reciprocals of the diagonal (not with !recips)
   const double* __restrict__ Ag = A + (size_t)sys * nnz;
   const double* Ig = init ? init + (size_t)sys * nnz : Ag;
   double anorm2 = 0.0;
@@ -199,15 +202,20 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
     double r2 = 0.0;
     const bool last = (it == sweeps);
     if (!TRACK && last) break;
-    if (FAST && !last) {
+    if ((FAST || recips) && !last) {
       // the correctly rounded reciprocal, the same value as 1.0 / u, by integer arithmetic (ifp::rcp): off
       // the FP64 unit, which the sweeps' FMAs and products keep busy
+      auto recip = [](double u) { return FAST ? ifp::rcp(u) : ifp::quot_rcp(u); };
 #pragma unroll
       for (int c = 0; c < CR; ++c)
-        if (tid + c * bd < P.n) rinv[tid + c * bd] = ifp::rcp(cur[rd[c]]);
-      for (int r = tid + CR * bd; r < P.n; r += bd) rinv[r] = ifp::rcp(cur[__ldg(P.diag + r)]);
+        if (tid + c * bd < P.n) rinv[tid + c * bd] = recip(cur[rd[c]]);
+      for (int r = tid + CR * bd; r < P.n; r += bd) rinv[r] = recip(cur[__ldg(P.diag + r)]);
       __syncthreads();
     }
+    auto ref_quot = [&](double a, int j) {
+      const double u = cur[__ldg(P.diag + j)];
+      return recips ? ifp::quot(a, u, rinv[j]) : ifp::quot_slow(a, u);
+    };
     // entries with dependency pairs (most pairs first, so a warp's lanes run
     // alike), read from the warp-blocked program: the words of a slot do not
     // depend on one another, so their loads overlap.  LOW (j < i) is a
@@ -228,7 +236,7 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
         if (last) return;
       }
       if constexpr (LOW)
-        nxt[k] = FAST ? as * rinv[j] : as / cur[__ldg(P.diag + j)];
+        nxt[k] = FAST ? as * rinv[j] : ref_quot(as, j);
       else
         nxt[k] = as;
     };
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
         r2 = fma(r, r, r2);
         if (last) return;
       }
-      nxt[k] = FAST ? a * rinv[j] : a / cur[__ldg(P.diag + j)];
+      nxt[k] = FAST ? a * rinv[j] : ref_quot(a, j);
     };
 #pragma unroll
     for (int c = 0; c < CL; ++c)
@@ -321,10 +329,14 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
 // FAST (BILU_REDUCE_FAST): the aiU entries are multiplied by the correctly
 // rounded reciprocal of the diagonal (ifp::rcp, one per row, the same value
 // as 1.0 / u) instead of divided -- one FP64 reciprocal per row instead of a
-// division per aiU entry.  The unit-diagonal aiL is unchanged.
+// division per aiU entry.  The unit-diagonal aiL is unchanged.  In the
+// reference order the quotients are formed from the same reciprocals
+// (ifp::quot: five FP64 instructions instead of a division's ten or so) where
+// they fit beside the values (recips; always, but for systems at the
+// shared-memory limit).
 template <typename FT, bool FAST>
 __global__ void __launch_bounds__(512) k_isai(const DevPattern P, int nsys, const double* __restrict__ LUg,
-                                              FT* __restrict__ ail, FT* __restrict__ aiu) {
+                                              FT* __restrict__ ail, FT* __restrict__ aiu, const int recips) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int sys = blockIdx.x;
   if (sys >= nsys) return;
@@ -357,16 +369,19 @@ __global__ void __launch_bounds__(512) k_isai(const DevPattern P, int nsys, cons
   for (int k = threadIdx.x; k < P.ail_nnz; k += blockDim.x) ail[(size_t)sys * P.ail_nnz + k] = (FT)M[k];
   __syncthreads();
   // ---- aiU
-  double* rinv = M + (P.ail_nnz > P.aiu_nnz ? P.ail_nnz : P.aiu_nnz);  // FAST: n reciprocals
-  if (FAST) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) rinv[i] = ifp::rcp(LU[__ldg(P.diag + i)]);
+  double* rinv = M + (P.ail_nnz > P.aiu_nnz ? P.ail_nnz : P.aiu_nnz);  // n reciprocals
+  if (FAST || recips) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const double u = LU[__ldg(P.diag + i)];
+      rinv[i] = FAST ? ifp::rcp(u) : ifp::quot_rcp(u);
+    }
     __syncthreads();
   }
   for (int sl = threadIdx.x; sl < n; sl += blockDim.x) {
     const int i = __ldg(P.aiu_perm + sl);
     const int beg = __ldg(P.aiu_rp + i), sz = __ldg(P.aiu_rp + i + 1) - beg;
     double* m = M + beg;
-    m[0] = FAST ? rinv[i] : 1.0 / LU[__ldg(P.diag + i)];
+    m[0] = FAST ? rinv[i] : ifp::rcp(LU[__ldg(P.diag + i)]);
     int q = __ldg(P.aiu_prog_ptr + (sl >> 5)) + (sl & 31);
     for (int blk = 1; blk < sz; ++blk) {
       const int h = __ldg(P.aiu_prog + q);  // t | count << 5; a row's words are 32 apart
@@ -379,7 +394,12 @@ __global__ void __launch_bounds__(512) k_isai(const DevPattern P, int nsys, cons
         acc = fma(-m[e & 31], LU[e >> 5], acc);
       }
       const int jt = __ldg(P.aiu_ci + beg + ht);
-      m[ht] = FAST ? acc * rinv[jt] : acc / LU[__ldg(P.diag + jt)];
+      if (FAST) {
+        m[ht] = acc * rinv[jt];
+      } else {
+        const double u = LU[__ldg(P.diag + jt)];
+        m[ht] = recips ? ifp::quot(acc, u, rinv[jt]) : ifp::quot_slow(acc, u);
+      }
     }
   }
   __syncthreads();
@@ -417,7 +437,7 @@ __device__ __forceinline__ float isai_block_f32(const int* __restrict__ prog, in
 // FP32 arithmetic); the FP64 pipe only rounds the factors.  No reference
 // counterpart (the library's definition; orc_isai_values_ex mode 2).
 __global__ void __launch_bounds__(512) k_isai_f32(const DevPattern P, int nsys, const double* __restrict__ LUg,
-                                                  float* __restrict__ ail, float* __restrict__ aiu) {
+                                                  float* __restrict__ ail, float* __restrict__ aiu, int) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int sys = blockIdx.x;
   if (sys >= nsys) return;
@@ -595,6 +615,9 @@ __global__ void k_to_sell(const int* __restrict__ src, int sell_nnz, int csr_nnz
   }
 }
 
+// whether a CTA may take `bytes` of dynamic shared memory beside 1 KB of static
+bool fits_smem(long long bytes) { return bytes + 1024 <= (long long)solve_max_smem(); }
+
 int grid_for(size_t total, int threads) {
   size_t g = (total + threads - 1) / threads;
   if (g > 65536) g = 65536;
@@ -624,7 +647,8 @@ cudaError_t launch_parilu0(const DevPattern& p, int nsys, const double* A, const
                            int sweeps, int threads, cudaStream_t st, double res_tol, int* sweeps_out,
                            double* res_out, int fast) {
   if (nsys == 0) return cudaSuccess;
-  const int smem = p.nnz * 8 * 2 + (fast ? p.n * 8 : 0);
+  const int recips = fast || fits_smem((long long)p.nnz * 16 + p.n * 8LL);
+  const int smem = p.nnz * 8 * 2 + (recips ? p.n * 8 : 0);
   const bool track = res_tol > 0.0 || res_out != nullptr;
   const bool small = threads <= 384;
   auto k = small ? (fast ? (track ? k_parilu0<true, true, true> : k_parilu0<true, false, true>)
@@ -633,7 +657,7 @@ cudaError_t launch_parilu0(const DevPattern& p, int nsys, const double* A, const
                          : (track ? k_parilu0<false, true, false> : k_parilu0<false, false, false>));
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  k<<<nsys, threads, smem, st>>>(p, nsys, A, init, lu, sweeps, res_tol, sweeps_out, res_out);
+  k<<<nsys, threads, smem, st>>>(p, nsys, A, init, lu, sweeps, res_tol, sweeps_out, res_out, recips);
   return cudaGetLastError();
 }
 
@@ -642,14 +666,15 @@ cudaError_t launch_isai(const DevPattern& p, int nsys, const double* lu, void* a
   if (nsys == 0) return cudaSuccess;
   const bool f32 = fp32 && fast && !p.l_diag;  // FAST FP32 ISAI: computed in FP32 (k_isai_f32)
   // k_isai_f32 stages the factors rounded to float; k_isai reads the FP64 factors through L1
-  const int smem = ((f32 ? p.nnz : 0) + (p.ail_nnz > p.aiu_nnz ? p.ail_nnz : p.aiu_nnz) + (fast ? p.n : 0)) *
-                   (f32 ? 4 : 8);
+  const int m = p.ail_nnz > p.aiu_nnz ? p.ail_nnz : p.aiu_nnz;
+  int recips = fast || fits_smem(8LL * (m + p.n));
+  const int smem = ((f32 ? p.nnz : 0) + m + (recips ? p.n : 0)) * (f32 ? 4 : 8);
   void* k = f32 ? (void*)k_isai_f32
                 : fp32 ? (fast ? (void*)k_isai<float, true> : (void*)k_isai<float, false>)
                        : (fast ? (void*)k_isai<double, true> : (void*)k_isai<double, false>);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  void* args[] = {const_cast<DevPattern*>(&p), &nsys, &lu, &ail, &aiu};
+  void* args[] = {const_cast<DevPattern*>(&p), &nsys, &lu, &ail, &aiu, &recips};
   return cudaLaunchKernel(k, dim3(nsys), dim3(threads), args, (size_t)smem, st);
 }
 

@@ -1,7 +1,8 @@
 // FP64 operations done exactly with integer arithmetic, bit for bit equal to
 // the hardware's: the FP64 <-> FP32 conversions (round to nearest even,
 // cvt.rn.f32.f64, and cvt.f64.f32) and the correctly rounded FP64 reciprocal
-// (__drcp_rn).
+// (__drcp_rn); and the correctly rounded quotient by a divisor whose
+// reciprocal is at hand.
 //
 // Why: GB300's FP64 unit is the bound of the factorisation and solver kernels
 // (about 1.6 FP64 FMAs per clock per SM), and these operations run there too;
@@ -146,6 +147,57 @@ __device__ __forceinline__ double rcp(double u) {
   double y = to_rcp(u, ok);
   if (!ok) y = rcp_slow(u);
   return y;
+}
+
+// Quotient by a divisor that is used several times: RN(a / u), the value of
+// a / u, from u and y = RN(1/u).
+//
+// Why: a division on GB300 issues 8 to 14 FP64-unit instructions (counted by
+// ncu in the kernels that use it), and the reference order divides by the same
+// u_jj many times: every iteration's upper solve, every lower entry of a
+// ParILU sweep, every aiU entry.  y comes from the integer pipes (rcp), so a
+// quotient costs five FP64 instructions (four with the tail yl of y).
+//
+// Method: P. Markstein's theorem (Computation of elementary functions on the
+// IBM RISC System/6000 processor, 1990): with y = RN(1/u) and q within one ulp
+// of a / u, r = a - u q is exact and RN(q + r y) is the correctly rounded
+// quotient.  RN(a y) alone can be 1.5 ulp off, so
+//   quot   corrects it once (q then differs from a / u by little more than
+//          half an ulp) and applies the theorem to the result;
+//   quot_t starts from a (y + yl), yl = (1 - u y) y, which is that close.
+// Both need operands away from the ends of the exponent range: |a| in
+// [2^-800, 2^801) and |u| in [2^-200, 2^201), where a / u and r stay normal.
+// quot_rcp returns NaN in the place of y for other u, and other a (0 among
+// them) fail the exponent test; both take the hardware's division in a call
+// that is not inlined.  bilu_check_integer_fp compares both with the division.
+__device__ __noinline__ double quot_slow(double a, double u) { return a / u; }
+
+__device__ __forceinline__ double quot_rcp(double u) {
+  const unsigned e = ((unsigned)__double2hiint(u) >> 20) & 0x7ffu;
+  return e - 823u <= 400u ? rcp(u) : __longlong_as_double(0x7ff8000000000000ll);
+}
+
+// the tail of quot_rcp(u) = y, for quot_t
+__device__ __forceinline__ double quot_tail(double u, double y) { return fma(-u, y, 1.0) * y; }
+
+__device__ __forceinline__ bool quot_ok(double a, double y) {
+  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu;
+  return ea - 223u <= 1600u && (__double2hiint(y) & 0x7ff00000) != 0x7ff00000;
+}
+
+__device__ __forceinline__ double quot(double a, double u, double y) {
+  const double p = a * y;
+  const double q = fma(fma(-u, p, a), y, p);
+  double v = fma(fma(-u, q, a), y, q);
+  if (!quot_ok(a, y)) v = quot_slow(a, u);
+  return v;
+}
+
+__device__ __forceinline__ double quot_t(double a, double u, double y, double yl) {
+  const double q = fma(a, y, a * yl);
+  double v = fma(fma(-u, q, a), y, q);
+  if (!quot_ok(a, y)) v = quot_slow(a, u);
+  return v;
 }
 
 }  // namespace

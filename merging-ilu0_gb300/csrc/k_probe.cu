@@ -121,6 +121,13 @@ __global__ void k_intfp_check(unsigned long long seed, int n, unsigned long long
     const double dv = __longlong_as_double((long long)v);
     const double ra = __drcp_rn(dv), rr = ifp::rcp(dv);
     if (__double_as_longlong(ra) != __double_as_longlong(rr) && !(ra != ra && rr != rr)) ++nr;
+    // quotients: any dividend by any divisor, then by one whose reciprocal has a tail of every size
+    const double div = (i & 1) ? dv : __longlong_as_double((long long)((v & 0x800fffffffffffffull) |
+                                                                       ((823ull + ((s >> 40) % 401u)) << 52)));
+    const double qy = ifp::quot_rcp(div), want = d / div;
+    const double q5 = ifp::quot(d, div, qy), q4 = ifp::quot_t(d, div, qy, ifp::quot_tail(div, qy));
+    if (__double_as_longlong(want) != __double_as_longlong(q5) && !(want != want && q5 != q5)) ++nr;
+    if (__double_as_longlong(want) != __double_as_longlong(q4) && !(want != want && q4 != q4)) ++nr;
   }
   if (nd) atomicAdd(bad, nd);
   if (nw) atomicAdd(bad + 1, nw);
