@@ -259,7 +259,10 @@ __host__ __device__ inline int rr_red_bytes(int nt) { return (2 * nt + 16) * 8; 
 // same on host and device: pv 0 none, 1 two-triangle ISAI, 2 general ISAI, 3
 // ILU factors (inkernel: the FP64 factorisation slot of the merged form).  The
 // reduction slot comes first, so the rest of the layout does not depend on nt.
-__host__ __device__ inline RRLayout rr_layout_base(int n, int nnz, int pv, bool fp32, bool inkernel, int nt) {
+// ref: the reference order, whose FP64 upper solve keeps three values per
+// diagonal (u, 1/u and its tail).
+__host__ __device__ inline RRLayout rr_layout_base(int n, int nnz, int pv, bool fp32, bool inkernel, int nt,
+                                                   bool ref = false) {
   RRLayout L;
   int off = 0;
   const int fts = fp32 ? 4 : 8;
@@ -273,7 +276,7 @@ __host__ __device__ inline RRLayout rr_layout_base(int n, int nnz, int pv, bool 
   if (pv == 1) take(L.mid, (long long)n * fts);
   if (pv == 3) {
     take(L.F, (long long)nnz * (inkernel ? 8 : fts));
-    take(L.rinv, (long long)n * fts);
+    take(L.rinv, (long long)n * fts * (ref && !fp32 ? 3 : 1));
   }
   L.total = off;
   return L;

@@ -333,7 +333,9 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
 // reference order the quotients are formed from the same reciprocals
 // (ifp::quot: five FP64 instructions instead of a division's ten or so) where
 // they fit beside the values (recips; always, but for systems at the
-// shared-memory limit).
+// shared-memory limit).  ifp::quot_t with the n tails beside them, one FP64
+// instruction less, is slower: they take L1 from the factors (ParILU(5) + ISAI
+// of 1024 3D 10x10x10 systems 451 against 423 us).
 template <typename FT, bool FAST>
 __global__ void __launch_bounds__(512) k_isai(const DevPattern P, int nsys, const double* __restrict__ LUg,
                                               FT* __restrict__ ail, FT* __restrict__ aiu, const int recips) {

@@ -9,12 +9,18 @@
 // partial sums are never -0 (fma(a, x, +0) is +0 when the product is zero),
 // so an addition of such a lane is an exact no-op and is skipped.  S = the
 // smallest power of two >= min(max row length, 32).
-template <int S, typename VT, typename IT>
+//
+// M = the longest row the instantiation serves (at most S): slots past it do
+// not exist, because an FMA or addition skipped under a lane's row length is
+// if-converted into a predicated one, which still takes its FP64-unit slot
+// (a 5-entry row in a 16-slot tree issues 31 FP64 instructions for the 9 it
+// needs).
+template <int S, int M = S, typename VT, typename IT>
 __device__ __forceinline__ double row_ref(const VT* __restrict__ a, const IT* __restrict__ ci, int beg, int L,
                                           const double* __restrict__ x) {
   double v[S];
 #pragma unroll
-  for (int l = 0; l < S; ++l) {
+  for (int l = 0; l < M; ++l) {
     double acc = 0.0;
     if (l < L) {
       acc = fma((double)a[beg + l], x[__ldg(ci + beg + l)], 0.0);
@@ -28,7 +34,7 @@ __device__ __forceinline__ double row_ref(const VT* __restrict__ a, const IT* __
   for (int off = S / 2; off >= 1; off >>= 1) {
 #pragma unroll
     for (int i = 0; i < off; ++i)
-      if (i + off < lc) v[i] += v[i + off];
+      if (i + off < M && i + off < lc) v[i] += v[i + off];
     lc = lc < off ? lc : off;
   }
   return v[0];

@@ -237,12 +237,14 @@ __device__ __forceinline__ void rows_acc_sell(const VT* __restrict__ val, const 
 // z_i into zd for FP32 factors.  Ends with a barrier.
 // REF: the reference's order instead (PrecondBiCGSTAB_exact_ilu0_app1_merged_gpu.cu:22-108):
 // s = sum of fma(F, y, s) from 0 in program order, then y_i - s, and for UPPER
-// (y_i - s) / u_ii with FP64 factors (rinv then holds u_ii itself) or
-// (y_i - s) * rinv_i with FP32 factors (the library's FP32 definition).
+// (y_i - s) / u_ii with FP64 factors or (y_i - s) * rinv_i with FP32 factors
+// (the library's FP32 definition).  The quotient is formed from the
+// reciprocal (ifp::quot_t: four FP64 instructions, the value of the division):
+// rinv then holds n diagonals, their n reciprocals and the n tails of these.
 template <bool UPPER, typename FT, bool REF>
 __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const int* __restrict__ prog, int nlev,
                                           const FT* __restrict__ F, const FT* __restrict__ rinv, FT* y, double* zd,
-                                          int tid, int nt, int maxcnt) {
+                                          int tid, int nt, int maxcnt, int n) {
   constexpr int PF = kTrsvPrefetch;
   // maxcnt: the most entries of any row of this triangle (the plan's
   // DevPattern::tp_maxcnt_*).  With FP64 factors, triangles whose rows have at
@@ -275,7 +277,11 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
       }
       const FT d = y[i] - acc;
       if (UPPER) {
-        const FT z = sizeof(FT) == 8 ? d / rinv[i] : d * rinv[i];
+        FT z;
+        if constexpr (sizeof(FT) == 8)
+          z = ifp::quot_t(d, rinv[i], rinv[n + i], rinv[2 * n + i]);
+        else
+          z = d * rinv[i];
         y[i] = z;
         if (sizeof(FT) == 4) zd[i] = (double)z;
       } else {
@@ -346,25 +352,39 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
 template <typename FT, bool REF>
 __device__ __forceinline__ void lu_apply(const DevPattern& P, const FT* __restrict__ F, const FT* __restrict__ rinv,
                                          FT* y, double* zd, int tid, int nt) {
-  tri_solve<false, FT, REF>(P.tp_lo_hdr, P.tp_lo, P.nlev_lo, F, rinv, y, zd, tid, nt, P.tp_maxcnt_lo);
-  tri_solve<true, FT, REF>(P.tp_up_hdr, P.tp_up, P.nlev_up, F, rinv, y, zd, tid, nt, P.tp_maxcnt_up);
+  tri_solve<false, FT, REF>(P.tp_lo_hdr, P.tp_lo, P.nlev_lo, F, rinv, y, zd, tid, nt, P.tp_maxcnt_lo, P.n);
+  tri_solve<true, FT, REF>(P.tp_up_hdr, P.tp_up, P.nlev_up, F, rinv, y, zd, tid, nt, P.tp_maxcnt_up, P.n);
 }
 
 // The reference-order SpMV rows (row_ref, the reference's warp-per-row tree
 // for rows of at most 16 entries) for this thread's rows, one row at a time.
-template <int R, typename VT, typename IT>
-__device__ __forceinline__ void rows_acc_ref(const VT* __restrict__ val, const IT* __restrict__ ci,
-                                             const int* __restrict__ rp, int tid, int nt, int n,
-                                             const double* __restrict__ xv, double (&out)[R]) {
+// maxl: the operator's longest row; rows of at most 5 and 7 entries (the 2D
+// 5-point and 3D 7-point stencils) have trees of just those slots.
+template <int S, int M, int R, typename VT, typename IT>
+__device__ __forceinline__ void rows_acc_ref_m(const VT* __restrict__ val, const IT* __restrict__ ci,
+                                               const int* __restrict__ rp, int tid, int nt, int n,
+                                               const double* __restrict__ xv, double (&out)[R]) {
 #pragma unroll
   for (int k = 0; k < R; ++k) {
     const int i = tid + k * nt;
     out[k] = 0.0;
     if (i < n) {
       const int beg = __ldg(rp + i);
-      out[k] = row_ref<16>(val, ci, beg, __ldg(rp + i + 1) - beg, xv);
+      out[k] = row_ref<S, M>(val, ci, beg, __ldg(rp + i + 1) - beg, xv);
     }
   }
+}
+
+template <int R, typename VT, typename IT>
+__device__ __forceinline__ void rows_acc_ref(const VT* __restrict__ val, const IT* __restrict__ ci,
+                                             const int* __restrict__ rp, int tid, int nt, int n,
+                                             const double* __restrict__ xv, double (&out)[R], int maxl) {
+  if (maxl <= 5)
+    rows_acc_ref_m<8, 5>(val, ci, rp, tid, nt, n, xv, out);
+  else if (maxl <= 7)
+    rows_acc_ref_m<8, 7>(val, ci, rp, tid, nt, n, xv, out);
+  else
+    rows_acc_ref_m<16, 16>(val, ci, rp, tid, nt, n, xv, out);
 }
 
 // PV: 0 none, 1 ISAI of L and U (z = aiU (aiL v)), 2 general ISAI (z = aiA v),
@@ -481,7 +501,14 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     __syncthreads();
     for (int i = tid; i < n; i += nt) {
       const double dgi = (double)Fs[__ldg(P.diag + i)];
-      rinv[i] = (REF && sizeof(FT) == 8) ? (FT)dgi : (FT)(1.0 / dgi);  // REF FP64 divides by u_ii
+      if (REF && sizeof(FT) == 8) {  // the upper solve's quotients by u_ii (tri_solve)
+        const double y = ifp::quot_rcp(dgi);
+        rinv[i] = (FT)dgi;
+        rinv[n + i] = (FT)y;
+        rinv[2 * n + i] = (FT)ifp::quot_tail(dgi, y);
+      } else {
+        rinv[i] = (FT)(1.0 / dgi);
+      }
     }
     // visible to the solves after the first reduction's barrier
   }
@@ -595,7 +622,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     BILU_RR_APPLY();  // p_hat in sph
     // v = A p_hat, (r_hat, v)
     if (REF)
-      rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, v);
+      rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, v, P.a_maxl);
     else if (Asell)
       rows_acc_sell<R>(Asell, saci, P.sa_off, arp, rb, rs, n, sph, v);
     else
@@ -637,7 +664,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     BILU_RR_APPLY();  // s_hat in sph
     // t = A s_hat, (t, s), (t, t)
     if (REF)
-      rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, t);
+      rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, t, P.a_maxl);
     else if (Asell)
       rows_acc_sell<R>(Asell, saci, P.sa_off, arp, rb, rs, n, sph, t);
     else
@@ -725,7 +752,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
       // inner product over i = 0 .. n-1.  Warp w holds rows 32 (w R + k) + l: it passes each
       // row's residual to every lane in row order, every lane runs the same FMA chain, and the
       // chain moves on to the next warp through red
-      rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, ax);
+      rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, ax, P.a_maxl);
       const int lane = tid & 31, warp = tid >> 5;
       double acc = 0.0;
       for (int w = 0; w < nw; ++w) {
