@@ -168,9 +168,10 @@ typedef struct bilu_plan_info {
                             occupancy variant of the register-resident kernel */
   int solver_kernel;     /* 0: one CTA per system, vectors in shared memory (every mode);
                             1: register-resident (BILU_REDUCE_FAST with n <= 1024, or
-                            the reference order with n <= 1024, ILU factors or none and
-                            rows of at most 16 entries): `threads` threads per system,
-                            each owning rows t + k * threads                         */
+                            ILU factors or none, rows of at most 16 entries and the
+                            reference order with n <= 1024 or either order with
+                            n <= 2048): `threads` threads per system, each owning at
+                            most 8 rows (FAST order with n <= 1024: t + k * threads) */
 } bilu_plan_info;
 bilu_status bilu_plan_get_info(const bilu_plan* plan, bilu_plan_info* info);
 

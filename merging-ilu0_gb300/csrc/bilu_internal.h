@@ -15,6 +15,10 @@ namespace bilu {
 // entries per row of a triangular-solve program that the register-resident
 // solver loads one level ahead (the rest it loads when it needs them)
 constexpr int kTrsvPrefetch = 4;
+// the programs' words: row | count << kTrsvShift and factor position <<
+// kTrsvShift | column, for systems of at most kRRMaxRows rows
+constexpr int kTrsvShift = 11;
+constexpr int kRRMaxRows = 1 << kTrsvShift;
 // op words per row of an ILU(0) program loaded one level ahead
 constexpr int kIluPrefetch = 16;
 
@@ -87,11 +91,13 @@ struct DevPattern {
   int nnz_L = 0, nnz_U = 0;
   const int* l_src = nullptr;
   const int* u_src = nullptr;
-  // triangular-solve programs of the register-resident solver (n <= 1024),
-  // one per triangle.  Level l: header {off, w}; at prog[off + s] the record
-  // of slot s < w, row | count << 10; at prog[off + w + j*w + s] its entry j,
-  // k << 10 | column, in summation order (lower ascending, upper descending k);
-  // every level has at least kTrsvPrefetch entry rows (padding reads as 0).
+  // triangular-solve programs of the register-resident solver (n <=
+  // kRRMaxRows), one per triangle.  Level l: header {off, w}; at prog[off + s]
+  // the record of slot s < w, row | count << kTrsvShift; at prog[off + w + j*w
+  // + s] its entry j, k << kTrsvShift | column, in summation order (lower
+  // ascending, upper descending k); every level has at least kTrsvPrefetch
+  // entry rows (padding reads as 0, but for the first entry of an upper row
+  // without entries, which holds its diagonal's k).
   const int2* tp_lo_hdr = nullptr;
   const int* tp_lo = nullptr;
   const int2* tp_up_hdr = nullptr;
@@ -234,7 +240,7 @@ __host__ __device__ inline SmemLayout layout_for(int n, int annz, int fnnz, int 
 }
 
 // Triangular-solve program of one triangle (DevPattern::tp_*) from its level
-// schedule (n <= 1024): header pairs {off, w} per level and the slot words.
+// schedule (n <= kRRMaxRows): header pairs {off, w} per level and the slot words.
 void build_trsv_program(const int* rp, const int* ci, const int* diag, const std::vector<int>& lptr,
                         const std::vector<int>& lrows, bool upper, std::vector<int>& hdr, std::vector<int>& prog);
 // ILU(0) program (DevPattern::ilu_*) of the factor pattern for one approach (1..4).
@@ -260,7 +266,7 @@ __host__ __device__ inline int rr_red_bytes(int nt) { return (2 * nt + 16) * 8; 
 // ILU factors (inkernel: the FP64 factorisation slot of the merged form).  The
 // reduction slot comes first, so the rest of the layout does not depend on nt.
 // ref: the reference order, whose FP64 upper solve keeps three values per
-// diagonal (u, 1/u and its tail).
+// diagonal (tri_solve; one for n > 1024).
 __host__ __device__ inline RRLayout rr_layout_base(int n, int nnz, int pv, bool fp32, bool inkernel, int nt,
                                                    bool ref = false) {
   RRLayout L;
@@ -276,7 +282,7 @@ __host__ __device__ inline RRLayout rr_layout_base(int n, int nnz, int pv, bool 
   if (pv == 1) take(L.mid, (long long)n * fts);
   if (pv == 3) {
     take(L.F, (long long)nnz * (inkernel ? 8 : fts));
-    take(L.rinv, (long long)n * fts * (ref && !fp32 ? 3 : 1));
+    take(L.rinv, (long long)n * fts * (ref && !fp32 && n <= 1024 ? 3 : 1));
   }
   L.total = off;
   return L;
@@ -317,10 +323,13 @@ cudaError_t launch_uneven(const UnevenArgs& u, int threads, int grid, int fp32, 
 cudaError_t launch_solve(const SolveArgs& a, int threads, int fp32, int reduce_fast, int maxl, cudaStream_t st);
 // register-resident solver: pv 0 none, 1 ISAI of L and U, 2 general ISAI, 3 ILU factors;
 // ref: the reference's operation order; occ: the occupancy variant (k_bicgstab_rr_occ: R = 2, 4, 8;
-// ILU factors at R = 2, 4)
+// ILU factors at R = 2, 4); nt: threads per system (more than 128 at R = 8: k_bicgstab_rr_wide)
 int rr_rows_per_thread(int n, int nt);  // smallest R in {1, 2, 4, 8} with R * nt >= n, else 0
-int rr_max_threads(int R);
-const void* rr_kernel(int pv, int fp32, int R, int ref, int occ);  // null: no such variant
+// the most threads per system at R rows per thread: wide (n > 1024; ILU factors or none) 256 at R = 8
+int rr_max_threads(int R, bool wide = false);
+const void* rr_kernel(int pv, int fp32, int R, int ref, int occ, int nt);  // null: no such variant
+// k_bicgstab_rr_wide (k_solve_rr_wide.cu)
+const void* rr_wide_kernel(int pv, int fp32, int ref, int nt);
 // the occupancy variant (k_bicgstab_rr_occ, k_solve_rr_occ.cu) for R rows per thread; null: none
 const void* rr_occ_kernel(int pv, int fp32, int R);
 cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int pv, int fp32, int ref, int occ,

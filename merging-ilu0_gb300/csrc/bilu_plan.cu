@@ -116,11 +116,12 @@ void build_trsv_program(const int* rp, const int* ci, const int* diag, const std
       const int i = lrows[lptr[l] + s];
       int j = 0;
       if (upper) {
-        for (int k = rp[i + 1] - 1; k > diag[i]; --k, ++j) prog[off + w + (size_t)j * w + s] = k << 10 | ci[k];
+        for (int k = rp[i + 1] - 1; k > diag[i]; --k, ++j) prog[off + w + (size_t)j * w + s] = k << kTrsvShift | ci[k];
       } else {
-        for (int k = rp[i]; k < diag[i]; ++k, ++j) prog[off + w + (size_t)j * w + s] = k << 10 | ci[k];
+        for (int k = rp[i]; k < diag[i]; ++k, ++j) prog[off + w + (size_t)j * w + s] = k << kTrsvShift | ci[k];
       }
-      prog[off + s] = i | j << 10;
+      prog[off + s] = i | j << kTrsvShift;
+      if (upper && j == 0) prog[off + w + s] = diag[i] << kTrsvShift;
     }
   }
 }
@@ -195,13 +196,13 @@ void build_levels(bilu_plan& P) {
 }
 
 // Triangular-solve programs (DevPattern::tp_*) from the level schedules; only
-// for n <= 1024 (10-bit rows and columns), the register-resident solver's range.
+// for the register-resident solver's range.
 void build_trsv_programs(bilu_plan& P) {
   P.tp_lo_hdr.clear();
   P.tp_lo.clear();
   P.tp_up_hdr.clear();
   P.tp_up.clear();
-  if (P.n > 1024) return;
+  if (P.n > kRRMaxRows || P.nnz >= (1 << (31 - kTrsvShift))) return;
   bilu::build_trsv_program(P.rp.data(), P.ci.data(), P.diag.data(), P.lev_lo_ptr, P.lev_lo_rows, false, P.tp_lo_hdr,
                            P.tp_lo);
   bilu::build_trsv_program(P.rp.data(), P.ci.data(), P.diag.data(), P.lev_up_ptr, P.lev_up_rows, true, P.tp_up_hdr,
@@ -405,14 +406,16 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
   const int n = P.n;
   nt = std::max(round_up(nt, 32), 32);
   const int R = rr_rows_per_thread(n, nt);
-  if (R == 0 || nt > rr_max_threads(R)) return false;
+  const bool wide = n > 1024;  // k_bicgstab_rr_wide, the shared-memory solver's bits in either order
+  if (R == 0 || nt > rr_max_threads(R, wide)) return false;
   const bool lu = (pk == PK_ILU_INKERNEL || pk == PK_LU_GLOBAL);
   const int pv = pk == PK_NONE ? 0 : (lu ? 3 : (P.general_isai ? 2 : 1));
   // Reference order: the inner products chain through the warps as the
   // reference's warp-0 sums; ILU factors or none (the ISAI solvers' serial
   // inner products stay on the shared-memory kernel), rows of at most 16
   // entries (row_ref<16>), no SELL-32 copies, no 4-CTA variant.
-  if (ref) {
+  // Systems of more than 1024 rows: the same restrictions in either order.
+  if (ref || wide) {
     if ((pv != 0 && pv != 3) || P.a_maxl > 16) return false;
     mask &= 7;
   }
@@ -435,7 +438,7 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
   cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
   cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const void* k = rr_kernel(pv, fp32 ? 1 : 0, R, ref ? 1 : 0, occ_variant ? 1 : 0);
+  const void* k = rr_kernel(pv, fp32 ? 1 : 0, R, ref ? 1 : 0, occ_variant ? 1 : 0, nt);
   if (!k) return false;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(optin, off)) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, nt, off) != cudaSuccess || occ < 1) {

@@ -18,7 +18,7 @@ __global__ void BILU_RR_BOUNDS k_bicgstab_rr(const SolveArgs a, const RRLayout L
   const int sys = blockIdx.x;
   if (sys >= a.nsys) return;
   const DevPattern& P = a.pat;
-  rr_solve<R, PV, FT, true, REF>(a, P, L, smem, sys, a.A + (size_t)sys * P.a_nnz, a.b + (size_t)sys * P.n,
+  rr_solve<R, PV, FT, true, REF ? kRef : kFast>(a, P, L, smem, sys, a.A + (size_t)sys * P.a_nnz, a.b + (size_t)sys * P.n,
                                  a.x + (size_t)sys * P.n);
 }
 
@@ -40,9 +40,13 @@ int rr_rows_per_thread(int n, int nt) {
   return 0;
 }
 
-int rr_max_threads(int R) { return R <= 1 ? 1024 : (R == 2 ? 512 : (R == 4 ? 256 : 128)); }
+int rr_max_threads(int R, bool wide) {
+  if (wide) return R == 8 ? 256 : 0;
+  return R <= 1 ? 1024 : (R == 2 ? 512 : (R == 4 ? 256 : 128));
+}
 
-const void* rr_kernel(int pv, int fp32, int R, int ref, int occ) {
+const void* rr_kernel(int pv, int fp32, int R, int ref, int occ, int nt) {
+  if (R == 8 && nt > 128) return occ ? nullptr : rr_wide_kernel(pv, fp32, ref, nt);
   if (occ) {  // FAST order, the occupancy variants (R = 2, 4, 8; ILU factors at R = 2, 4)
     if (ref || (R != 2 && R != 4 && R != 8) || (R == 8 && pv == 3)) return nullptr;
     return rr_occ_kernel(pv, fp32, R);
@@ -62,8 +66,8 @@ cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int p
                             cudaStream_t st) {
   if (a.nsys == 0) return cudaSuccess;
   const int R = rr_rows_per_thread(a.pat.n, nt);
-  if (R == 0 || nt % 32 || nt > rr_max_threads(R)) return cudaErrorInvalidConfiguration;
-  const void* k = rr_kernel(pv, fp32, R, ref, occ);
+  if (R == 0 || nt % 32 || nt > rr_max_threads(R, a.pat.n > 1024)) return cudaErrorInvalidConfiguration;
+  const void* k = rr_kernel(pv, fp32, R, ref, occ, nt);
   if (!k) return cudaErrorInvalidConfiguration;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total);
   if (e != cudaSuccess) return e;

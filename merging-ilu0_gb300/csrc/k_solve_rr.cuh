@@ -226,26 +226,57 @@ __device__ __forceinline__ void rows_acc_sell(const VT* __restrict__ val, const 
   }
 }
 
-// One triangle of z = U^{-1} L^{-1} y over the CTA, level by level, in place
-// on y, from the triangle's solve program (DevPattern::tp_*).  Thread t takes
-// slot t of every level (and t + nt, ... of wider ones); the record and the
-// first kTrsvPrefetch entries of its next slot are loaded one level ahead and
-// the level headers two levels ahead, so the global-memory latency of the
-// program overlaps the current level's arithmetic and barrier.
+// The orders a solver instantiation follows.
+//   kFast    the FAST order (top of this file)
+//   kRef     the reference's operation order
+//   kFastChain  the FAST order of systems past the FAST kernels' 1024 rows,
+//            the shared-memory solver's (k_solve.cu with REF = false): rows and
+//            reciprocals as in FAST, triangular-solve sums, inner products and
+//            the true residual's rows as in the reference
+enum RROrder : int { kFast = 0, kRef = 1, kFastChain = 2 };
+
+// Barrier at the end of a level.  WIDE: of the solve's `team` threads, one
+// warp per 32 rows of the widest level (a warp barrier for one warp); the other
+// warps wait once, at the end of the apply.  Otherwise of the CTA: with one
+// CTA of at most four warps per system, a choice of the team in these kernels
+// costs more than the idle warps do (a second copy of the solves: 3D
+// 10x10x10 6.26 -> 6.66 ms, uneven batches 3.33 -> 3.69 ms; a branch per
+// level: 6.53 and 3.45 ms).
+template <bool WIDE>
+__device__ __forceinline__ void team_sync(int team) {
+  if (!WIDE)
+    __syncthreads();
+  else if (team <= 32)
+    __syncwarp();
+  else
+    asm volatile("bar.sync 1, %0;" ::"r"(team) : "memory");
+}
+
+// One triangle of z = U^{-1} L^{-1} y, level by level, in place on y, from the
+// triangle's solve program (DevPattern::tp_*), by the first `team` threads of
+// the CTA.  Thread t takes slot t of every level (and t + team, ... of wider
+// ones); the record and the first kTrsvPrefetch entries of its next slot are
+// loaded one level ahead and the level headers two levels ahead, so the
+// global-memory latency of the program overlaps the current level's
+// arithmetic and barrier.
 // Row i starts from y_i and subtracts its products in program order (one FMA
 // each, no separate subtraction); UPPER then scales by rinv_i and also widens
-// z_i into zd for FP32 factors.  Ends with a barrier.
-// REF: the reference's order instead (PrecondBiCGSTAB_exact_ilu0_app1_merged_gpu.cu:22-108):
+// z_i into zd for FP32 factors.  Ends with the team's barrier.
+// ORD != kFast: the reference's order instead (PrecondBiCGSTAB_exact_ilu0_app1_merged_gpu.cu:22-108):
 // s = sum of fma(F, y, s) from 0 in program order, then y_i - s, and for UPPER
-// (y_i - s) / u_ii with FP64 factors or (y_i - s) * rinv_i with FP32 factors
-// (the library's FP32 definition).  The quotient is formed from the
-// reciprocal (ifp::quot_t: four FP64 instructions, the value of the division):
-// rinv then holds n diagonals, their n reciprocals and the n tails of these.
-template <bool UPPER, typename FT, bool REF>
+// (y_i - s) / u_ii (kRef with FP64 factors) or (y_i - s) * rinv_i (FP32
+// factors and kFastChain, the library's definitions).  The quotient is formed
+// from the reciprocal (the value of the division, k_intfp.cuh): rinv holds n
+// reciprocals, their n tails and the n u_ii (four FP64 instructions).  WIDE
+// keeps the reciprocals alone (five FP64 instructions, 20 KB less): u_ii is
+// the factor just before the row's upper entries, and where the row has none
+// the program's first entry holds its position.
+template <bool UPPER, typename FT, int ORD, bool WIDE>
 __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const int* __restrict__ prog, int nlev,
                                           const FT* __restrict__ F, const FT* __restrict__ rinv, FT* y, double* zd,
-                                          int tid, int nt, int maxcnt, int n) {
+                                          int tid, int team, int maxcnt, int n) {
   constexpr int PF = kTrsvPrefetch;
+  constexpr int SH = kTrsvShift, MASK = (1 << kTrsvShift) - 1;
   // maxcnt: the most entries of any row of this triangle (the plan's
   // DevPattern::tp_maxcnt_*).  With FP64 factors, triangles whose rows have at
   // most two entries (5-point stencils) run a copy of the row code with two
@@ -259,29 +290,31 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
   // use the FP32 pipe, and the second copy cost the FP32 3D solve 4 %).
   const bool two = sizeof(FT) == 8 && maxcnt <= 2;
   auto row = [&](int rec, const int (&e)[PF], int off, int w, int s) {
-    const int i = rec & 1023, cnt = rec >> 10;
-    if (REF) {
+    const int i = rec & MASK, cnt = rec >> SH;
+    if (ORD != kFast) {
       FT acc = FT(0);
       if (two) {
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-          if (j < cnt) acc = fma_t(F[e[j] >> 10], y[e[j] & 1023], acc);
+          if (j < cnt) acc = fma_t(F[e[j] >> SH], y[e[j] & MASK], acc);
       } else {
 #pragma unroll
         for (int j = 0; j < PF; ++j)
-          if (j < cnt) acc = fma_t(F[e[j] >> 10], y[e[j] & 1023], acc);
+          if (j < cnt) acc = fma_t(F[e[j] >> SH], y[e[j] & MASK], acc);
       }
       for (int j = PF; j < cnt; ++j) {
         const int en = __ldg(prog + off + w + j * w + s);
-        acc = fma_t(F[en >> 10], y[en & 1023], acc);
+        acc = fma_t(F[en >> SH], y[en & MASK], acc);
       }
       const FT d = y[i] - acc;
       if (UPPER) {
         FT z;
-        if constexpr (sizeof(FT) == 8)
-          z = ifp::quot_t(d, rinv[i], rinv[n + i], rinv[2 * n + i]);
-        else
+        if constexpr (sizeof(FT) == 8 && ORD == kRef) {
+          z = WIDE ? ifp::quot(d, F[(e[0] >> SH) - cnt], rinv[i])
+                   : ifp::quot_t(d, rinv[2 * n + i], rinv[i], rinv[n + i]);
+        } else {
           z = d * rinv[i];
+        }
         y[i] = z;
         if (sizeof(FT) == 4) zd[i] = (double)z;
       } else {
@@ -293,15 +326,15 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
     if (two) {
 #pragma unroll
       for (int j = 0; j < 2; ++j)
-        if (j < cnt) acc = fma_t(-F[e[j] >> 10], y[e[j] & 1023], acc);
+        if (j < cnt) acc = fma_t(-F[e[j] >> SH], y[e[j] & MASK], acc);
     } else {
 #pragma unroll
       for (int j = 0; j < PF; ++j)
-        if (j < cnt) acc = fma_t(-F[e[j] >> 10], y[e[j] & 1023], acc);
+        if (j < cnt) acc = fma_t(-F[e[j] >> SH], y[e[j] & MASK], acc);
     }
     for (int j = PF; j < cnt; ++j) {
       const int en = __ldg(prog + off + w + j * w + s);
-      acc = fma_t(-F[en >> 10], y[en & 1023], acc);
+      acc = fma_t(-F[en >> SH], y[en & MASK], acc);
     }
     if (UPPER) {
       const FT z = acc * rinv[i];
@@ -329,14 +362,14 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
     int recn, en[PF];
     fetch(hn, recn, en);
     if (tid < h.y) row(rec, e, h.x, h.y, tid);
-    for (int s = tid + nt; s < h.y; s += nt) {
+    for (int s = tid + team; s < h.y; s += team) {
       int r2, e2[PF];
       r2 = __ldg(prog + h.x + s);
 #pragma unroll
       for (int j = 0; j < PF; ++j) e2[j] = __ldg(prog + h.x + h.y + j * h.y + s);
       row(r2, e2, h.x, h.y, s);
     }
-    __syncthreads();
+    team_sync<WIDE>(team);
     h = hn;
     hn = hnn;
     rec = recn;
@@ -345,15 +378,19 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
   }
 }
 
-// z = U^{-1} L^{-1} y over the CTA (y: the preconditioner input, already
-// rounded to FT; for FP64 factors y is the FP64 SpMV input itself, for FP32
-// factors the upper solve widens z into zd).  Ends with a barrier: z is
-// visible to every thread.
-template <typename FT, bool REF>
+// z = U^{-1} L^{-1} y (y: the preconditioner input, already rounded to FT; for
+// FP64 factors y is the FP64 SpMV input itself, for FP32 factors the upper
+// solve widens z into zd).  Ends with a CTA barrier: z is visible to every
+// thread.
+template <typename FT, int ORD, bool WIDE>
 __device__ __forceinline__ void lu_apply(const DevPattern& P, const FT* __restrict__ F, const FT* __restrict__ rinv,
                                          FT* y, double* zd, int tid, int nt) {
-  tri_solve<false, FT, REF>(P.tp_lo_hdr, P.tp_lo, P.nlev_lo, F, rinv, y, zd, tid, nt, P.tp_maxcnt_lo, P.n);
-  tri_solve<true, FT, REF>(P.tp_up_hdr, P.tp_up, P.nlev_up, F, rinv, y, zd, tid, nt, P.tp_maxcnt_up, P.n);
+  const int team = WIDE ? min(nt, (max(max(P.maxw_lo, P.maxw_up), 1) + 31) & ~31) : nt;
+  if (tid < team) {
+    tri_solve<false, FT, ORD, WIDE>(P.tp_lo_hdr, P.tp_lo, P.nlev_lo, F, rinv, y, zd, tid, team, P.tp_maxcnt_lo, P.n);
+    tri_solve<true, FT, ORD, WIDE>(P.tp_up_hdr, P.tp_up, P.nlev_up, F, rinv, y, zd, tid, team, P.tp_maxcnt_up, P.n);
+  }
+  if (WIDE) __syncthreads();
 }
 
 // The reference-order SpMV rows (row_ref, the reference's warp-per-row tree
@@ -403,10 +440,11 @@ __device__ __forceinline__ auto pick_ci(const unsigned short* c16, const int* c3
 // Solves system `sys` (result slot) with the CTA: P its pattern, L its
 // shared-memory carve-up, Ag / bg / xg its values, right-hand side and
 // solution.  Block-wide.
-template <int R, int PV, typename FT, bool C16, bool REF>
+template <int R, int PV, typename FT, bool C16, int ORD, bool WIDE = false>
 __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P, const RRLayout& L,
                                          unsigned char* smem, const int sys, const double* Ag, const double* bg,
                                          double* xg) {
+  constexpr bool REF = ORD != kFast;  // inner products in the reference's order, row blocks to match
   const int n = P.n, nt = blockDim.x, tid = threadIdx.x, nw = nt >> 5;
   // this thread's rows: rb + k * rs, k < R.  FAST: tid + k * nt.  REF: lane +
   // 32 (warp R + k), so that a warp's rows are a block of the reference's
@@ -501,11 +539,13 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     __syncthreads();
     for (int i = tid; i < n; i += nt) {
       const double dgi = (double)Fs[__ldg(P.diag + i)];
-      if (REF && sizeof(FT) == 8) {  // the upper solve's quotients by u_ii (tri_solve)
+      if (ORD == kRef && sizeof(FT) == 8) {  // the upper solve's quotients by u_ii (tri_solve)
         const double y = ifp::quot_rcp(dgi);
-        rinv[i] = (FT)dgi;
-        rinv[n + i] = (FT)y;
-        rinv[2 * n + i] = (FT)ifp::quot_tail(dgi, y);
+        rinv[i] = (FT)y;
+        if (!WIDE) {
+          rinv[n + i] = (FT)ifp::quot_tail(dgi, y);
+          rinv[2 * n + i] = (FT)dgi;
+        }
       } else {
         rinv[i] = (FT)(1.0 / dgi);
       }
@@ -592,7 +632,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
       }                                                                                                          \
       __syncthreads();                                                                                           \
     } else if (PV == 3) {                                                                                        \
-      lu_apply<FT, REF>(P, Fs, rinv, sizeof(FT) == 8 ? reinterpret_cast<FT*>(sph) : sin, sph, tid, nt);         \
+      lu_apply<FT, ORD, WIDE>(P, Fs, rinv, sizeof(FT) == 8 ? reinterpret_cast<FT*>(sph) : sin, sph, tid, nt);         \
     }                                                                                                            \
   } while (0)
 // writes this thread's rows of `vec` as the preconditioner input
@@ -621,7 +661,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     __syncthreads();
     BILU_RR_APPLY();  // p_hat in sph
     // v = A p_hat, (r_hat, v)
-    if (REF)
+    if (ORD == kRef)
       rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, v, P.a_maxl);
     else if (Asell)
       rows_acc_sell<R>(Asell, saci, P.sa_off, arp, rb, rs, n, sph, v);
@@ -663,7 +703,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     }
     BILU_RR_APPLY();  // s_hat in sph
     // t = A s_hat, (t, s), (t, t)
-    if (REF)
+    if (ORD == kRef)
       rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, t, P.a_maxl);
     else if (Asell)
       rows_acc_sell<R>(Asell, saci, P.sa_off, arp, rb, rs, n, sph, t);
@@ -753,6 +793,15 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
       // row's residual to every lane in row order, every lane runs the same FMA chain, and the
       // chain moves on to the next warp through red
       rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, ax, P.a_maxl);
+      if (ORD == kFastChain) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+          const int i = rb + k * rs;
+          r[k] = i < n ? __ldg(bg + i) - ax[k] : 0.0;
+        }
+        if (ref_chain_sum<1, R>(q, t_bb, red, nw) && lane0) a.true_res[sys] = sqrt(q[0]);
+        return;
+      }
       const int lane = tid & 31, warp = tid >> 5;
       double acc = 0.0;
       for (int w = 0; w < nw; ++w) {
@@ -791,6 +840,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
   }
 }
 
+// 8 rows per thread: 3 CTAs of 128 threads per SM
 #define BILU_RR_BOUNDS __launch_bounds__(R <= 1 ? 1024 : (R == 2 ? 512 : (R == 4 ? 256 : 128)), R == 8 ? 3 : 1)
 
 }  // namespace

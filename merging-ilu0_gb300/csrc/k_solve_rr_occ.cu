@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(OccBounds<R, PV>::threads, OccBounds<R, PV>::c
   const int sys = blockIdx.x;
   if (sys >= a.nsys) return;
   const DevPattern& P = a.pat;
-  rr_solve<R, PV, FT, true, false>(a, P, L, smem, sys, a.A + (size_t)sys * P.a_nnz, a.b + (size_t)sys * P.n,
+  rr_solve<R, PV, FT, true, kFast>(a, P, L, smem, sys, a.A + (size_t)sys * P.a_nnz, a.b + (size_t)sys * P.n,
                                    a.x + (size_t)sys * P.n);
 }
 

@@ -52,7 +52,7 @@ __global__ void BILU_RR_BOUNDS k_bicgstab_rr_uneven(const UnevenArgs u) {
       P.ilu_prog_approach = u.base.approach;
     }
     const RRLayout L = rr_layout_base(d.n, d.nnz, PV, sizeof(FT) == 4, true, blockDim.x);
-    rr_solve<R, PV, FT, false, false>(u.base, P, L, smem, sys, u.base.A + d.val_off, u.base.b + d.vec_off,
+    rr_solve<R, PV, FT, false, kFast>(u.base, P, L, smem, sys, u.base.A + d.val_off, u.base.b + d.vec_off,
                                       u.base.x + d.vec_off);
     if (!queue) break;
     __syncthreads();  // every thread is done with this system (shared memory, the slot)
