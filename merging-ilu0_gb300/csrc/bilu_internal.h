@@ -19,6 +19,10 @@ constexpr int kTrsvPrefetch = 4;
 // kTrsvShift | column, for systems of at most kRRMaxRows rows
 constexpr int kTrsvShift = 11;
 constexpr int kRRMaxRows = 1 << kTrsvShift;
+// compact solve programs: factor positions below 2^17, and the bit that marks
+// a slot as used
+constexpr int kCompactMaxNnz = 1 << 17;
+constexpr unsigned kCompactUsed = 1u << 30;
 // op words per row of an ILU(0) program loaded one level ahead
 constexpr int kIluPrefetch = 16;
 
@@ -105,6 +109,15 @@ struct DevPattern {
   // the most entries of any row of the lower / upper solve program (the
   // solves run no product slot past it); kTrsvPrefetch when not known
   int tp_maxcnt_lo = kTrsvPrefetch, tp_maxcnt_up = kTrsvPrefetch;
+  // compact solve programs, where every row of both triangles has at most three
+  // entries (tc_mc = 2 or 3: the most; 0: none): level l is the maxw_lo (maxw_up)
+  // words from l * maxw_lo, one per slot; a word holds the row (bits 0-10), its
+  // entries (11-12), the first one's factor position (13-29; a lower row's
+  // entries follow it, an upper row's precede it), the used bit (30), and the
+  // columns from bit 32, 11 bits each but for the third one's top bit (31)
+  const uint2* tc_lo = nullptr;
+  const uint2* tc_up = nullptr;
+  int tc_mc = 0;
   // ILU(0) program of the register-resident solver's merged form (n <= 1024),
   // per lower level: header {off, w, len, 0}; slot s word j at prog[off + j*w + s]:
   // word 0 = number of op words that follow; ops per entry k of the row in
@@ -323,13 +336,16 @@ cudaError_t launch_uneven(const UnevenArgs& u, int threads, int grid, int fp32, 
 cudaError_t launch_solve(const SolveArgs& a, int threads, int fp32, int reduce_fast, int maxl, cudaStream_t st);
 // register-resident solver: pv 0 none, 1 ISAI of L and U, 2 general ISAI, 3 ILU factors;
 // ref: the reference's operation order; occ: the occupancy variant (k_bicgstab_rr_occ: R = 2, 4, 8;
-// ILU factors at R = 2, 4); nt: threads per system (more than 128 at R = 8: k_bicgstab_rr_wide)
+// ILU factors at R = 2, 4); nt: threads per system (more than 128 at R = 8: k_bicgstab_rr_wide);
+// mc: DevPattern::tc_mc (ILU factors; ignored by the occupancy variants)
 int rr_rows_per_thread(int n, int nt);  // smallest R in {1, 2, 4, 8} with R * nt >= n, else 0
 // the most threads per system at R rows per thread: wide (n > 1024; ILU factors or none) 256 at R = 8
 int rr_max_threads(int R, bool wide = false);
-const void* rr_kernel(int pv, int fp32, int R, int ref, int occ, int nt);  // null: no such variant
+const void* rr_kernel(int pv, int fp32, int R, int ref, int occ, int nt, int mc);  // null: no such variant
+// k_bicgstab_rr_lu (k_solve_rr_lu.cu)
+const void* rr_lu_kernel(int fp32, int R, int ref, int mc);
 // k_bicgstab_rr_wide (k_solve_rr_wide.cu)
-const void* rr_wide_kernel(int pv, int fp32, int ref, int nt);
+const void* rr_wide_kernel(int pv, int fp32, int ref, int nt, int mc);
 // the occupancy variant (k_bicgstab_rr_occ, k_solve_rr_occ.cu) for R rows per thread; null: none
 const void* rr_occ_kernel(int pv, int fp32, int R);
 cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int pv, int fp32, int ref, int occ,
@@ -402,6 +418,8 @@ struct bilu_plan {
   std::vector<int> l_rp, l_ci, l_src, u_rp, u_ci, u_src;
   std::vector<int> row_lev, tpos, mlp_ent;
   std::vector<int> tp_lo_hdr, tp_lo, tp_up_hdr, tp_up;  // triangular-solve programs (DevPattern::tp_*)
+  std::vector<int> tc_lo, tc_up;                         // compact solve programs (DevPattern::tc_*)
+  int tc_mc = 0;
   std::vector<int> ilu_hdr, ilu_prog;                    // ILU(0) program (DevPattern::ilu_*)
   std::vector<int> sa_off, sa_ci, sa_src, su_off, su_ci, su_src;  // SELL-32 layouts (DevPattern::sa_*, su_*)
   std::vector<int> pl_ent;  // ParILU entry classes (see DevPattern::pl_ent)

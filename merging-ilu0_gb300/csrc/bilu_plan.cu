@@ -195,6 +195,38 @@ void build_levels(bilu_plan& P) {
                        P.lev_up_ptr, P.lev_up_rows, P.maxw_up);
 }
 
+// Compact solve programs (DevPattern::tc_*), where no row of either triangle
+// has more than three entries.  Their levels are all as wide as the widest one,
+// so a schedule whose levels fill less than a quarter of that keeps the general
+// programs (padding would crowd the words out of L1).
+void build_compact_programs(bilu_plan& P) {
+  P.tc_lo.clear();
+  P.tc_up.clear();
+  P.tc_mc = 0;
+  int mc = 0;
+  for (int i = 0; i < P.n; ++i) mc = std::max({mc, P.diag[i] - P.rp[i], P.rp[i + 1] - 1 - P.diag[i]});
+  const long long slots_lo = (long long)(P.lev_lo_ptr.size() - 1) * P.maxw_lo;
+  const long long slots_up = (long long)(P.lev_up_ptr.size() - 1) * P.maxw_up;
+  if (mc > 3 || P.nnz >= kCompactMaxNnz || std::max(slots_lo, slots_up) > 4LL * P.n) return;
+  auto fill = [&](const std::vector<int>& ptr, const std::vector<int>& rows, int W, bool upper, std::vector<int>& out) {
+    out.assign(2 * (ptr.size() - 1) * (size_t)W, 0);
+    for (size_t l = 0; l + 1 < ptr.size(); ++l)
+      for (int q = ptr[l]; q < ptr[l + 1]; ++q) {
+        const int i = rows[q];
+        const int cnt = upper ? P.rp[i + 1] - 1 - P.diag[i] : P.diag[i] - P.rp[i];
+        const int k0 = upper ? P.rp[i + 1] - 1 : P.rp[i];
+        unsigned c[3] = {0, 0, 0};
+        for (int j = 0; j < cnt; ++j) c[j] = (unsigned)P.ci[upper ? k0 - j : k0 + j];
+        unsigned* w = reinterpret_cast<unsigned*>(out.data()) + 2 * (l * W + (q - ptr[l]));
+        w[0] = (unsigned)i | (unsigned)cnt << 11 | (unsigned)k0 << 13 | kCompactUsed | (c[2] >> 10) << 31;
+        w[1] = c[0] | c[1] << 11 | c[2] << 22;
+      }
+  };
+  fill(P.lev_lo_ptr, P.lev_lo_rows, P.maxw_lo, false, P.tc_lo);
+  fill(P.lev_up_ptr, P.lev_up_rows, P.maxw_up, true, P.tc_up);
+  P.tc_mc = std::max(mc, 2);
+}
+
 // Triangular-solve programs (DevPattern::tp_*) from the level schedules; only
 // for the register-resident solver's range.
 void build_trsv_programs(bilu_plan& P) {
@@ -207,6 +239,7 @@ void build_trsv_programs(bilu_plan& P) {
                            P.tp_lo);
   bilu::build_trsv_program(P.rp.data(), P.ci.data(), P.diag.data(), P.lev_up_ptr, P.lev_up_rows, true, P.tp_up_hdr,
                            P.tp_up);
+  build_compact_programs(P);
 }
 
 // SELL-32 layout of a pattern with n <= 1024 rows (DevPattern::sa_* / su_*).
@@ -438,7 +471,7 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
   cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
   cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const void* k = rr_kernel(pv, fp32 ? 1 : 0, R, ref ? 1 : 0, occ_variant ? 1 : 0, nt);
+  const void* k = rr_kernel(pv, fp32 ? 1 : 0, R, ref ? 1 : 0, occ_variant ? 1 : 0, nt, P.tc_mc);
   if (!k) return false;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(optin, off)) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, nt, off) != cudaSuccess || occ < 1) {
@@ -498,6 +531,7 @@ bilu_status upload(bilu_plan& P) {
   const size_t o_plent = put(P.pl_ent);
   const size_t o_plpp = put(P.pl_prog_ptr), o_plp = put(P.pl_prog);
   const size_t o_tlh = put(P.tp_lo_hdr), o_tl = put(P.tp_lo), o_tuh = put(P.tp_up_hdr), o_tu = put(P.tp_up);
+  const size_t o_tcl = put(P.tc_lo), o_tcu = put(P.tc_up);
   const size_t o_sao = put(P.sa_off), o_sac = put(P.sa_ci), o_sas = put(P.sa_src);
   const size_t o_ih = put(P.ilu_hdr), o_ip = put(P.ilu_prog);
   // 16-bit column indices, two per int
@@ -641,6 +675,11 @@ bilu_status upload(bilu_plan& P) {
     }
     d.tp_maxcnt_lo = ml;
     d.tp_maxcnt_up = mu;
+  }
+  if (P.tc_mc) {
+    d.tc_lo = reinterpret_cast<const uint2*>(b + o_tcl);
+    d.tc_up = reinterpret_cast<const uint2*>(b + o_tcu);
+    d.tc_mc = P.tc_mc;
   }
   d.pl_ndep = P.pl_ndep;
   d.pl_nlow = P.pl_nlow;

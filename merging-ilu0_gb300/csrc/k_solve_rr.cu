@@ -45,8 +45,9 @@ int rr_max_threads(int R, bool wide) {
   return R <= 1 ? 1024 : (R == 2 ? 512 : (R == 4 ? 256 : 128));
 }
 
-const void* rr_kernel(int pv, int fp32, int R, int ref, int occ, int nt) {
-  if (R == 8 && nt > 128) return occ ? nullptr : rr_wide_kernel(pv, fp32, ref, nt);
+const void* rr_kernel(int pv, int fp32, int R, int ref, int occ, int nt, int mc) {
+  if (R == 8 && nt > 128) return occ ? nullptr : rr_wide_kernel(pv, fp32, ref, nt, mc);
+  if (pv == 3 && mc && !occ) return rr_lu_kernel(fp32, R, ref, mc);
   if (occ) {  // FAST order, the occupancy variants (R = 2, 4, 8; ILU factors at R = 2, 4)
     if (ref || (R != 2 && R != 4 && R != 8) || (R == 8 && pv == 3)) return nullptr;
     return rr_occ_kernel(pv, fp32, R);
@@ -67,7 +68,7 @@ cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int p
   if (a.nsys == 0) return cudaSuccess;
   const int R = rr_rows_per_thread(a.pat.n, nt);
   if (R == 0 || nt % 32 || nt > rr_max_threads(R, a.pat.n > 1024)) return cudaErrorInvalidConfiguration;
-  const void* k = rr_kernel(pv, fp32, R, ref, occ, nt);
+  const void* k = rr_kernel(pv, fp32, R, ref, occ, nt, a.pat.tc_mc);
   if (!k) return cudaErrorInvalidConfiguration;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total);
   if (e != cudaSuccess) return e;

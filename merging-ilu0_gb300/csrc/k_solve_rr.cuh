@@ -378,17 +378,81 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
   }
 }
 
+// tri_solve from the triangle's compact program (DevPattern::tc_*; rows of at
+// most MC = 2 or 3 entries, the 2D 5-point and 3D 7-point stencils): the same
+// operations in the same order.  Measured against the general program: see the
+// kernels that use it (k_solve_rr_lu.cu, k_solve_rr_wide.cu).  A slot is one
+// 64-bit word instead of five 32-bit ones and there are no level headers (a
+// level is W slots, the unused ones marked), so the words of the next DEPTH
+// levels fit in registers and the loop loads one word per level; and no
+// product slot past MC is issued, which predicated off still takes its
+// FP64-unit slot.
+template <bool UPPER, typename FT, int ORD, bool WIDE, int MC>
+__device__ __forceinline__ void tri_solve_compact(const uint2* __restrict__ prog, int W, int nlev,
+                                                  const FT* __restrict__ F, const FT* __restrict__ rinv, FT* y,
+                                                  double* zd, int tid, int team, int n) {
+  constexpr int DEPTH = WIDE ? 4 : 2;
+  constexpr unsigned M = kRRMaxRows - 1;
+  auto row = [&](uint2 w) {
+    const int i = w.x & M, cnt = (w.x >> 11) & 3, k0 = (w.x >> 13) & (kCompactMaxNnz - 1);
+    int c[3];
+    c[0] = w.y & M;
+    c[1] = (w.y >> 11) & M;
+    c[2] = MC == 3 ? (w.y >> 22) | (WIDE ? (w.x >> 31) << 10 : 0u) : 0;
+    FT acc = ORD != kFast ? FT(0) : y[i];
+#pragma unroll
+    for (int j = 0; j < MC; ++j)
+      if (j < cnt) {
+        const FT f = F[UPPER ? k0 - j : k0 + j];
+        acc = fma_t(ORD != kFast ? f : -f, y[c[j]], acc);
+      }
+    if (ORD != kFast) acc = y[i] - acc;
+    if (UPPER) {
+      if constexpr (sizeof(FT) == 8 && ORD == kRef)
+        acc = WIDE ? ifp::quot(acc, F[k0 - cnt], rinv[i]) : ifp::quot_t(acc, rinv[2 * n + i], rinv[i], rinv[n + i]);
+      else
+        acc = acc * rinv[i];
+      if (sizeof(FT) == 4) zd[i] = (double)acc;
+    }
+    y[i] = acc;
+  };
+  const uint2 none = make_uint2(0u, 0u);
+  uint2 q[DEPTH];
+  const uint2* p = prog + tid;
+#pragma unroll
+  for (int d = 0; d < DEPTH; ++d) q[d] = tid < W && d < nlev ? __ldg(p + d * W) : none;
+  for (int lev = 0; lev < nlev; ++lev) {
+    const uint2 next = tid < W && lev + DEPTH < nlev ? __ldg(p + DEPTH * W) : none;
+    if (q[0].x & kCompactUsed) row(q[0]);
+    for (int s = team; s < W - tid; s += team) {
+      const uint2 w = __ldg(p + s);
+      if (w.x & kCompactUsed) row(w);
+    }
+    team_sync<WIDE>(team);
+    p += W;
+#pragma unroll
+    for (int d = 0; d + 1 < DEPTH; ++d) q[d] = q[d + 1];
+    q[DEPTH - 1] = next;
+  }
+}
+
 // z = U^{-1} L^{-1} y (y: the preconditioner input, already rounded to FT; for
 // FP64 factors y is the FP64 SpMV input itself, for FP32 factors the upper
-// solve widens z into zd).  Ends with a CTA barrier: z is visible to every
-// thread.
-template <typename FT, int ORD, bool WIDE>
+// solve widens z into zd).  MC: 0, the general programs, else the compact ones.
+// Ends with a CTA barrier: z is visible to every thread.
+template <typename FT, int ORD, bool WIDE, int MC>
 __device__ __forceinline__ void lu_apply(const DevPattern& P, const FT* __restrict__ F, const FT* __restrict__ rinv,
                                          FT* y, double* zd, int tid, int nt) {
   const int team = WIDE ? min(nt, (max(max(P.maxw_lo, P.maxw_up), 1) + 31) & ~31) : nt;
-  if (tid < team) {
-    tri_solve<false, FT, ORD, WIDE>(P.tp_lo_hdr, P.tp_lo, P.nlev_lo, F, rinv, y, zd, tid, team, P.tp_maxcnt_lo, P.n);
-    tri_solve<true, FT, ORD, WIDE>(P.tp_up_hdr, P.tp_up, P.nlev_up, F, rinv, y, zd, tid, team, P.tp_maxcnt_up, P.n);
+  if (!WIDE || tid < team) {
+    if constexpr (MC > 0) {
+      tri_solve_compact<false, FT, ORD, WIDE, MC>(P.tc_lo, P.maxw_lo, P.nlev_lo, F, rinv, y, zd, tid, team, P.n);
+      tri_solve_compact<true, FT, ORD, WIDE, MC>(P.tc_up, P.maxw_up, P.nlev_up, F, rinv, y, zd, tid, team, P.n);
+    } else {
+      tri_solve<false, FT, ORD, WIDE>(P.tp_lo_hdr, P.tp_lo, P.nlev_lo, F, rinv, y, zd, tid, team, P.tp_maxcnt_lo,
+                                      P.n);
+      tri_solve<true, FT, ORD, WIDE>(P.tp_up_hdr, P.tp_up, P.nlev_up, F, rinv, y, zd, tid, team, P.tp_maxcnt_up, P.n);
+    }
   }
   if (WIDE) __syncthreads();
 }
@@ -440,7 +504,7 @@ __device__ __forceinline__ auto pick_ci(const unsigned short* c16, const int* c3
 // Solves system `sys` (result slot) with the CTA: P its pattern, L its
 // shared-memory carve-up, Ag / bg / xg its values, right-hand side and
 // solution.  Block-wide.
-template <int R, int PV, typename FT, bool C16, int ORD, bool WIDE = false>
+template <int R, int PV, typename FT, bool C16, int ORD, bool WIDE = false, int MC = 0>
 __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P, const RRLayout& L,
                                          unsigned char* smem, const int sys, const double* Ag, const double* bg,
                                          double* xg) {
@@ -632,7 +696,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
       }                                                                                                          \
       __syncthreads();                                                                                           \
     } else if (PV == 3) {                                                                                        \
-      lu_apply<FT, ORD, WIDE>(P, Fs, rinv, sizeof(FT) == 8 ? reinterpret_cast<FT*>(sph) : sin, sph, tid, nt);         \
+      lu_apply<FT, ORD, WIDE, MC>(P, Fs, rinv, sizeof(FT) == 8 ? reinterpret_cast<FT*>(sph) : sin, sph, tid, nt);         \
     }                                                                                                            \
   } while (0)
 // writes this thread's rows of `vec` as the preconditioner input
