@@ -131,10 +131,11 @@ def solver_kernel_name(info, n, opts):
     rows = next(r for r in (1, 2, 4, 8) if r * info["threads"] >= n)
     pv = {0: 3, 1: 3, 2: 3, 3: 1, 4: 1, 5: 0, 6: 2}[opts["precond"]]
     ft = "float" if opts.get("factor_precision", 0) == 1 and pv else "double"
-    if info["operands_in_smem"] & 16:
+    if info["operands_in_smem"] & 16 and rows < 8:
         return f"k_bicgstab_rr_occ<{rows}, {pv}, {ft}> (register-resident solver, occupancy variant, " \
                f"{info['threads']} threads per system)"
-    return f"k_bicgstab_rr<{rows}, {pv}, {ft}> (register-resident solver, {info['threads']} threads per system)"
+    split = ", on k_bicgstab_rr_split" if rows == 8 and pv != 3 and opts.get("reduction", 0) == 1 else ""
+    return f"k_bicgstab_rr<{rows}, {pv}, {ft}> (register-resident solver, {info['threads']} threads per system{split})"
 
 
 def launches_per_step(info):

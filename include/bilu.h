@@ -111,10 +111,11 @@ typedef struct bilu_options {
                                 SELL-32 copies made before the solver launch (same
                                 arithmetic; the copies live in the plan's workspace).
                                 Bit 4: the kernel variant bounded for occupancy (same
-                                arithmetic, fewer registers, more threads per SM): 8 rows
-                                per thread on 4 CTAs of 128 threads per SM, 4 rows on 4
-                                CTAs of 256 (3 with ILU factors), 2 rows on 2 CTAs of
-                                512; ignored for ILU factors at 8 rows per thread.        */
+                                arithmetic, fewer registers, more threads per SM): 3 or 4
+                                rows per thread on 4 CTAs of 256 (3 with ILU factors), 2
+                                rows on 2 CTAs of 512; ignored for ILU factors at 5 to 8
+                                rows per thread; without them those rows always run on
+                                two or four threads per system thread, same arithmetic.   */
 } bilu_options;
 
 /* Fills *opts with the reference defaults: merged ILU(0), approach 1, 5 sweeps,

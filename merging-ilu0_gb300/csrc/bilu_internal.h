@@ -270,8 +270,8 @@ struct RRLayout {
   int red = -1, ph = -1, in = -1, mid = -1, F = -1, rinv = -1, A = -1, ail = -1, aiu = -1, total = 0;
 };
 
-// Bytes of the reduction slot of an nt-thread CTA: two partial sums per
-// thread and 16 broadcast scalars.
+// Bytes of the reduction slot of a system whose order has nt threads: two
+// partial sums per order thread and 16 broadcast scalars.
 __host__ __device__ inline int rr_red_bytes(int nt) { return (2 * nt + 16) * 8; }
 
 // The mandatory part of an RRLayout (no optional staging) for nt threads, the
@@ -334,22 +334,21 @@ void* uneven_kernel(int fp32, int reduce_fast, int maxl);
 cudaError_t launch_uneven(const UnevenArgs& u, int threads, int grid, int fp32, int reduce_fast, int maxl,
                           cudaStream_t st);
 cudaError_t launch_solve(const SolveArgs& a, int threads, int fp32, int reduce_fast, int maxl, cudaStream_t st);
-// register-resident solver: pv 0 none, 1 ISAI of L and U, 2 general ISAI, 3 ILU factors;
-// ref: the reference's operation order; occ: the occupancy variant (k_bicgstab_rr_occ: R = 2, 4, 8;
-// ILU factors at R = 2, 4); nt: threads per system (more than 128 at R = 8: k_bicgstab_rr_wide);
-// mc: DevPattern::tc_mc (ILU factors; ignored by the occupancy variants)
+// register-resident solver: pv 0 none, 1 ISAI of L and U, 2 general ISAI, 3 ILU factors; ref: the reference's
+// operation order; nt: the order's threads per system; occ: the occupancy variant (k_bicgstab_rr_occ, 2 to 4 rows
+// per thread, FAST order); mc: DevPattern::tc_mc
 int rr_rows_per_thread(int n, int nt);  // smallest R in {1, 2, 4, 8} with R * nt >= n, else 0
+int rr_slots(int n, int nt);            // the row slots of the kernels: 3 and 6 too
 // the most threads per system at R rows per thread: wide (n > 1024; ILU factors or none) 256 at R = 8
 int rr_max_threads(int R, bool wide = false);
-const void* rr_kernel(int pv, int fp32, int R, int ref, int occ, int nt, int mc);  // null: no such variant
-// k_bicgstab_rr_lu (k_solve_rr_lu.cu)
-const void* rr_lu_kernel(int fp32, int R, int ref, int mc);
-// k_bicgstab_rr_wide (k_solve_rr_wide.cu)
-const void* rr_wide_kernel(int pv, int fp32, int ref, int nt, int mc);
-// the occupancy variant (k_bicgstab_rr_occ, k_solve_rr_occ.cu) for R rows per thread; null: none
-const void* rr_occ_kernel(int pv, int fp32, int R);
+int rr_split(int pv, int ref, int n, int nt, int nsys, int nsm);  // threads per order thread of a batch
+const void* rr_kernel(int pv, int fp32, int n, int nt, int ref, int occ, int mc, int split);  // null: no such variant
+const void* rr_wide_kernel(int pv, int fp32, int ref, int nt, int mc);      // k_solve_rr_wide.cu
+const void* rr_split_kernel(int pv, int fp32, int split, int slots);        // k_solve_rr_split.cu
+const void* rr_lu_kernel(int fp32, int slots, int ref, int mc);             // k_solve_rr_lu.cu
+const void* rr_occ_kernel(int pv, int fp32, int slots);                     // k_solve_rr_occ.cu
 cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int pv, int fp32, int ref, int occ,
-                            cudaStream_t st);
+                            int nsm, cudaStream_t st);
 size_t solve_max_smem();
 cudaError_t launch_expand(const DevPattern& p, int nsys, const double* vin, double* vout, cudaStream_t st);
 cudaError_t launch_ilu0(const DevPattern& p, int nsys, const double* A, double* lu, int approach, int threads,
@@ -440,7 +439,8 @@ struct bilu_plan {
   bool rr = false;
   int rr_threads = 0, rr_pv = 0;
   bool rr_sell = false;  // SpMVs read SELL-32 copies of A (and of aiU) made before the solver launch
-  bool rr_occ = false;  // the 4-CTAs-per-SM kernel variant (staging bit 4)
+  bool rr_occ = false;   // the occupancy variant was asked for (staging bit 4)
+  int nsm = 0;           // SMs of the device
   bilu::RRLayout rr_lay;
   // workspace
   void* ws = nullptr;

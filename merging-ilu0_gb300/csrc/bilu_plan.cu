@@ -428,9 +428,9 @@ void choose_layout(bilu_plan& P) {
 // operands that would cost occupancy are left in global memory, read through
 // L1; ILU factors are always staged; bit 3: the SpMVs read SELL-32 copies of
 // the operands left in global memory; bit 4: the occupancy variant of the
-// kernel (k_bicgstab_rr_occ: 8 rows per thread on 4 CTAs of 128 threads, 4 rows
-// on 4 CTAs of 256 (3 with ILU factors), 2 rows on 2 CTAs of 512; ignored for
-// ILU factors at 8 rows per thread); false when the kernel does not apply or
+// kernel (k_bicgstab_rr_occ: 4 rows on 4 CTAs of 256 (3 with ILU factors), 2
+// rows on 2 CTAs of 512; ignored for ILU factors at 5 to 8 rows per thread, and
+// without them those have just one kernel, k_bicgstab_rr_split); false when the kernel does not apply or
 // that configuration is invalid.
 bool rr_configure(bilu_plan& P, int nt, int mask) {
   const bilu_options& o = P.opts;
@@ -460,6 +460,8 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
   const int fts = fp32 ? 4 : 8;
   if (pv == 3 && P.tp_lo.empty()) return false;
   // the merged form factorises in FP64 in the factor slot before rounding to FT
+  // more systems than are resident at once; fewer may run on more threads (rr_split) with the same layout
+  const int split = rr_split(pv, ref ? 1 : 0, n, nt, 1 << 30, P.nsm);
   RRLayout L = rr_layout_base(n, P.nnz, pv, fp32, pk == PK_ILU_INKERNEL, nt, ref);
   int off = L.total;
   auto take = [&](int& dst, long long bytes) {
@@ -471,10 +473,10 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
   cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
   cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const void* k = rr_kernel(pv, fp32 ? 1 : 0, R, ref ? 1 : 0, occ_variant ? 1 : 0, nt, P.tc_mc);
+  const void* k = rr_kernel(pv, fp32 ? 1 : 0, n, nt, ref ? 1 : 0, occ_variant && split == 1 ? 1 : 0, P.tc_mc, split);
   if (!k) return false;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(optin, off)) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, nt, off) != cudaSuccess || occ < 1) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, nt * split, off) != cudaSuccess || occ < 1) {
     cudaGetLastError();
     return false;
   }
@@ -498,18 +500,22 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
 
 // Default: the caller's threads per system, else the fewest warps that give
 // every thread at most 8 rows (one warp for n <= 256); the caller's staging
-// mask, else the ISAI values but not A; SELL-32 copies for ILU factors at
-// n > 512.  Measured on GB300 (3D 7-point 10x10x10, 7x7x7, 2D 16x16): A read
-// through L1 beats A in shared memory, whose carve-out shrinks the L1 left for
-// the column indices and ISAI values; the FP32 aiL in shared memory helps when
-// it fits; the SELL-32 copy of A gains 5 % with ILU factors at 10x10x10
-// (128 threads) and loses up to 6 % on the smaller systems and with ISAI.
+// mask, else SELL-32 copies for ILU factors at n > 512, the ISAI values in
+// shared memory at up to 4 rows per thread and nothing at 5 to 8.  Measured on
+// GB300 (3D 7-point 10x10x10, 7x7x7, 2D 16x16): A read through L1 beats A in
+// shared memory, whose carve-out shrinks the L1 left for the column indices
+// and ISAI values; so do the ISAI values at 5 to 8 rows (k_bicgstab_rr_split,
+// FP32 ISAI of 4096 3D 10x10x10 systems: 3.52 ms, with aiL and aiU in shared
+// memory 4.82; within 1 % at 7x7x7, 16x16 and 23x25); the SELL-32 copy of A
+// gains 5 % with ILU factors at 10x10x10 (128 threads) and loses up to 6 % on
+// the smaller systems and with ISAI.
 void choose_rr(bilu_plan& P) {
   const bilu_options& o = P.opts;
   P.rr = false;
   int nt = o.threads_per_system > 0 ? o.threads_per_system : round_up((P.n + 7) / 8, 32);
   const bool lu = prec_kind(o.precond) == PK_ILU_INKERNEL || prec_kind(o.precond) == PK_LU_GLOBAL;
-  rr_configure(P, nt, o.smem_staging >= 0 ? o.smem_staging : (6 | (lu && P.n > 512 ? 8 : 0)));
+  const bool split = rr_split(lu ? 3 : 1, o.reduction != BILU_REDUCE_FAST, P.n, nt, 1 << 30, P.nsm) > 1;
+  rr_configure(P, nt, o.smem_staging >= 0 ? o.smem_staging : ((split ? 0 : 6) | (lu && P.n > 512 ? 8 : 0)));
 }
 
 bilu_status upload(bilu_plan& P) {
@@ -809,6 +815,7 @@ bilu_status bilu_plan_create(bilu_plan** out, int n, int nnz, const int* h_rp, c
   else
     bilu_default_options(&P->opts);
   cudaGetDevice(&P->device);
+  cudaDeviceGetAttribute(&P->nsm, cudaDevAttrMultiProcessorCount, P->device);
   P->n = n;
   P->nnz_in = nnz;
   P->in_rp.assign(h_rp, h_rp + n + 1);
@@ -996,7 +1003,7 @@ bilu_status bilu_plan_autotune(bilu_plan* P, int nsys, const double* d_values, c
   for (int f : {1, 2, 4}) {
     for (int mask : {0, 2, 6, 1, 8, 10, 14, 16, 18, 22, 24, 26}) {
       const int rf = rr_rows_per_thread(P->n, base * f);
-      if ((mask & 16) && (rf < 2 || (rf == 8 && P->rr_pv == 3))) continue;  // bit 4 ignored
+      if ((mask & 16) && (rf < 2 || rf == 8)) continue;  // bit 4 ignored, or the same kernel
       if ((mask & 24) && P->opts.reduction != BILU_REDUCE_FAST) continue;                         // bits 3, 4 ignored
       if (!rr_configure(*P, base * f, mask)) continue;
       float ms = 0.0f;
@@ -1228,7 +1235,7 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
     a.A_sell = (const double*)(ws + sc.asell);
   }
   e = P->rr ? launch_solve_rr(a, P->rr_lay, P->rr_threads, P->rr_pv, fp32 ? 1 : 0,
-                              o.reduction == BILU_REDUCE_FAST ? 0 : 1, P->rr_occ ? 1 : 0, st)
+                              o.reduction == BILU_REDUCE_FAST ? 0 : 1, P->rr_occ ? 1 : 0, P->nsm, st)
             : launch_solve(a, P->threads, fp32 ? 1 : 0, o.reduction == BILU_REDUCE_FAST ? 1 : 0, maxl, st);
   if (e != cudaSuccess) return cuda_err(e, "solver launch");
   if (P->timing) cudaEventRecord(P->ev[2], st);

@@ -23,13 +23,16 @@ __global__ void BILU_RR_BOUNDS k_bicgstab_rr(const SolveArgs a, const RRLayout L
 }
 
 template <int PV, typename FT, bool REF>
-const void* rr_kernel_pv(int R) {
-  switch (R) {
+const void* rr_kernel_pv(int slots) {
+  switch (slots) {
     case 1: return (const void*)k_bicgstab_rr<1, PV, FT, REF>;
     case 2: return (const void*)k_bicgstab_rr<2, PV, FT, REF>;
+    case 3: return (const void*)k_bicgstab_rr<3, PV, FT, REF>;
     case 4: return (const void*)k_bicgstab_rr<4, PV, FT, REF>;
-    default: return (const void*)k_bicgstab_rr<8, PV, FT, REF>;
   }
+  if constexpr (PV == 3 || REF)  // else split (rr_split)
+    return slots == 6 ? (const void*)k_bicgstab_rr<6, PV, FT, REF> : (const void*)k_bicgstab_rr<8, PV, FT, REF>;
+  return nullptr;
 }
 
 }  // namespace
@@ -40,40 +43,61 @@ int rr_rows_per_thread(int n, int nt) {
   return 0;
 }
 
+int rr_slots(int n, int nt) {
+  for (int R : {1, 2, 3, 4, 6, 8})
+    if ((long long)R * nt >= n) return R;
+  return 0;
+}
+
 int rr_max_threads(int R, bool wide) {
   if (wide) return R == 8 ? 256 : 0;
   return R <= 1 ? 1024 : (R == 2 ? 512 : (R == 4 ? 256 : 128));
 }
 
-const void* rr_kernel(int pv, int fp32, int R, int ref, int occ, int nt, int mc) {
-  if (R == 8 && nt > 128) return occ ? nullptr : rr_wide_kernel(pv, fp32, ref, nt, mc);
-  if (pv == 3 && mc && !occ) return rr_lu_kernel(fp32, R, ref, mc);
-  if (occ) {  // FAST order, the occupancy variants (R = 2, 4, 8; ILU factors at R = 2, 4)
-    if (ref || (R != 2 && R != 4 && R != 8) || (R == 8 && pv == 3)) return nullptr;
-    return rr_occ_kernel(pv, fp32, R);
-  }
-  if (ref) {  // reference order: no preconditioner or ILU factors (one warp per system)
-    if (pv == 0) return rr_kernel_pv<0, double, true>(R);
-    if (pv == 3) return fp32 ? rr_kernel_pv<3, float, true>(R) : rr_kernel_pv<3, double, true>(R);
+// Threads per order thread (k_bicgstab_rr_split): FAST order without ILU
+// factors at 5 to 8 rows per thread.  Four while every system then is resident
+// at once (64 registers: 1024 threads per SM), where a system's own latency is
+// all that counts: 16 systems of 3D 10x10x10, FP32 ISAI, 0.375 ms on one, 0.336
+// on two, 0.246 on four; 300 systems 0.495 / 0.449 / 0.352; 450, which four
+// leave waiting, 0.543 / 0.474 / 0.580.  Past that two, but for 7 or 8 rows on
+// one warp (8192 2D 16x16 systems 1.64 ms on two, 1.47 on four; at 96 and 128
+// threads four are 5 to 15 % slower).
+int rr_split(int pv, int ref, int n, int nt, int nsys, int nsm) {
+  const int slots = rr_slots(n, nt);
+  if (pv == 3 || ref || slots < 6 || nt > 128) return 1;
+  if (nsys <= (long long)nsm * (1024 / (4 * nt))) return 4;
+  return slots == 8 && nt == 32 ? 4 : 2;
+}
+
+const void* rr_kernel(int pv, int fp32, int n, int nt, int ref, int occ, int mc, int split) {
+  const int slots = rr_slots(n, nt);
+  if (nt > 128 && slots > 4) return occ ? nullptr : rr_wide_kernel(pv, fp32, ref, nt, mc);
+  if (split > 1) return rr_split_kernel(pv, fp32, split, slots);
+  if (occ) return ref ? nullptr : rr_occ_kernel(pv, fp32, slots);  // FAST order, 2 to 4 rows
+  if (pv == 3 && mc) return rr_lu_kernel(fp32, slots, ref, mc);
+  if (ref) {  // reference order: no preconditioner or ILU factors
+    if (pv == 0) return rr_kernel_pv<0, double, true>(slots);
+    if (pv == 3) return fp32 ? rr_kernel_pv<3, float, true>(slots) : rr_kernel_pv<3, double, true>(slots);
     return nullptr;
   }
-  if (pv == 0) return rr_kernel_pv<0, double, false>(R);
-  if (pv == 1) return fp32 ? rr_kernel_pv<1, float, false>(R) : rr_kernel_pv<1, double, false>(R);
-  if (pv == 3) return fp32 ? rr_kernel_pv<3, float, false>(R) : rr_kernel_pv<3, double, false>(R);
-  return fp32 ? rr_kernel_pv<2, float, false>(R) : rr_kernel_pv<2, double, false>(R);
+  if (pv == 0) return rr_kernel_pv<0, double, false>(slots);
+  if (pv == 1) return fp32 ? rr_kernel_pv<1, float, false>(slots) : rr_kernel_pv<1, double, false>(slots);
+  if (pv == 3) return fp32 ? rr_kernel_pv<3, float, false>(slots) : rr_kernel_pv<3, double, false>(slots);
+  return fp32 ? rr_kernel_pv<2, float, false>(slots) : rr_kernel_pv<2, double, false>(slots);
 }
 
 cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int pv, int fp32, int ref, int occ,
-                            cudaStream_t st) {
+                            int nsm, cudaStream_t st) {
   if (a.nsys == 0) return cudaSuccess;
   const int R = rr_rows_per_thread(a.pat.n, nt);
   if (R == 0 || nt % 32 || nt > rr_max_threads(R, a.pat.n > 1024)) return cudaErrorInvalidConfiguration;
-  const void* k = rr_kernel(pv, fp32, R, ref, occ, nt, a.pat.tc_mc);
+  const int split = rr_split(pv, ref, a.pat.n, nt, a.nsys, nsm);
+  const void* k = rr_kernel(pv, fp32, a.pat.n, nt, ref, occ, a.pat.tc_mc, split);
   if (!k) return cudaErrorInvalidConfiguration;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<SolveArgs*>(&a), const_cast<RRLayout*>(&L)};
-  return cudaLaunchKernel(k, dim3(a.nsys), dim3(nt), args, (size_t)L.total, st);
+  return cudaLaunchKernel(k, dim3(a.nsys), dim3(nt * split), args, (size_t)L.total, st);
 }
 
 }  // namespace bilu

@@ -152,6 +152,59 @@ __device__ __forceinline__ bool ref_chain_sum(double (&v)[K], Term term, double*
   return true;
 }
 
+// The FAST order of nto threads per system run by SPLIT * nto threads: thread
+// h * nto + t owns the h-th part of order thread t's rows, R of them, so the
+// chain of t's partial passes from part to part through red, and the last part
+// sums the partials as block_sum_w0 does for nto threads.  Returns true on the
+// last part's first warp, which forms the scalar recurrence and broadcasts it.
+template <int K, int R, int SPLIT, bool LANES_FIRST, typename Term>
+__device__ __forceinline__ bool split_chain_sum(double (&v)[K], Term term, double* red, int nto, int h, int t) {
+  const int lane = threadIdx.x & 31, warp = t >> 5, nw = nto >> 5;
+#pragma unroll
+  for (int s = 0; s < SPLIT; ++s) {
+    if (h == s) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) v[j] = s == 0 ? 0.0 : red[j * nto + t];
+#pragma unroll
+      for (int k = 0; k < R; ++k) term(k, v);
+      if (s + 1 < SPLIT || LANES_FIRST) {
+#pragma unroll
+        for (int j = 0; j < K; ++j) red[j * nto + t] = v[j];
+      }
+    }
+    if (s + 1 < SPLIT) __syncthreads();
+  }
+  if (h != SPLIT - 1) return false;
+  if (!LANES_FIRST) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+#pragma unroll
+      for (int off = 16; off >= 1; off >>= 1) v[j] = v[j] + __shfl_xor_sync(kFull, v[j], off);
+    }
+  }
+  if (nw > 1) {
+    if (!LANES_FIRST) {  // the partials have been read: their slots take the warps' sums
+      asm volatile("bar.sync 1, %0;" ::"r"(nto) : "memory");
+#pragma unroll
+      for (int j = 0; j < K; ++j)
+        if (lane == 0) red[j * nto + warp] = v[j];
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(nto) : "memory");
+  }
+  if (warp != 0) return false;
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    double s = LANES_FIRST ? (nw > 1 ? red[j * nto + lane] : v[j]) : v[j];
+    for (int w = 1; w < nw; ++w) s = s + red[j * nto + (LANES_FIRST ? w * 32 + lane : w)];
+    if (LANES_FIRST) {
+#pragma unroll
+      for (int off = 16; off >= 1; off >>= 1) s = s + __shfl_xor_sync(kFull, s, off);
+    }
+    v[j] = s;
+  }
+  return true;
+}
+
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 // FP64 -> FT and FT -> FP64 with the integer conversions for float (k_intfp.cuh).
@@ -504,17 +557,20 @@ __device__ __forceinline__ auto pick_ci(const unsigned short* c16, const int* c3
 // Solves system `sys` (result slot) with the CTA: P its pattern, L its
 // shared-memory carve-up, Ag / bg / xg its values, right-hand side and
 // solution.  Block-wide.
-template <int R, int PV, typename FT, bool C16, int ORD, bool WIDE = false, int MC = 0>
+template <int R, int PV, typename FT, bool C16, int ORD, bool WIDE = false, int MC = 0, int SPLIT = 1>
 __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P, const RRLayout& L,
                                          unsigned char* smem, const int sys, const double* Ag, const double* bg,
                                          double* xg) {
   constexpr bool REF = ORD != kFast;  // inner products in the reference's order, row blocks to match
   const int n = P.n, nt = blockDim.x, tid = threadIdx.x, nw = nt >> 5;
-  // this thread's rows: rb + k * rs, k < R.  FAST: tid + k * nt.  REF: lane +
-  // 32 (warp R + k), so that a warp's rows are a block of the reference's
-  // lane-strided inner-product terms (ref_chain_sum)
-  const int rb = REF ? (tid & 31) + 32 * R * (tid >> 5) : tid;
-  const int rs = REF ? 32 : nt;
+  // this thread's rows: rb + k * rs, k < R.  FAST: tid + k * nt, split: the h-th
+  // part of order thread t's (split_chain_sum).  REF: lane + 32 (warp R + k), so
+  // that a warp's rows are a block of the reference's lane-strided
+  // inner-product terms (ref_chain_sum)
+  constexpr bool CHAIN = REF || SPLIT > 1;  // inner products pass from warp to warp (term by term) through red
+  const int nto = nt / SPLIT, h = SPLIT > 1 ? tid / nto : 0, t_ord = tid - h * nto;
+  const int rb = REF ? (tid & 31) + 32 * R * (tid >> 5) : t_ord + h * R * nto;
+  const int rs = REF ? 32 : nto;
   const int* __restrict__ arp = P.a_rp;
   const auto* __restrict__ aci = pick_ci<C16>(P.a_ci16, P.a_ci);
   const auto* __restrict__ lci = pick_ci<C16>(P.ail_ci16, P.ail_ci);
@@ -522,7 +578,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
   const auto* __restrict__ saci = pick_ci<C16>(P.sa_ci16, P.sa_ci);
   const auto* __restrict__ suci = pick_ci<C16>(P.su_ci16, P.su_ci);
 
-  double* red = reinterpret_cast<double*>(smem + L.red);  // 2 partials per thread, then 16 broadcast scalars
+  double* red = reinterpret_cast<double*>(smem + L.red);  // 2 partials per order thread, then 16 broadcast scalars
   double* sph = reinterpret_cast<double*>(smem + L.ph);
   FT* sin = reinterpret_cast<FT*>(smem + L.in);
   FT* smid = reinterpret_cast<FT*>(smem + L.mid);
@@ -634,13 +690,15 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
   }
   // ||b||^2 = (r, r_hat) at the start: one reduction serves both (its barrier
   // also completes the staging above).  bc: the scalars warp 0 broadcasts.
-  double* bc = red + 2 * nt;
+  double* bc = red + 2 * nto;
   const bool lane0 = (tid & 31) == 0;
   // the CTA's sum of q (and of its second slot for K = 2): FAST, the block
   // reduction of the thread partials; REF, the reference's chain over the
   // rows, term(k, acc) per row
-#define BILU_RR_SUM(K, qv, TERM) \
-  (REF ? ref_chain_sum<K, R>(qv, TERM, red, nw) : block_sum_w0<K, PV != 3>(qv, red, nw))
+#define BILU_RR_SUM(K, qv, TERM)                                                                      \
+  (REF         ? ref_chain_sum<K, R>(qv, TERM, red, nw)                                               \
+   : SPLIT > 1 ? split_chain_sum<K, R, SPLIT, PV != 3>(qv, TERM, red, nto, h, t_ord)                  \
+               : block_sum_w0<K, PV != 3>(qv, red, nw))
   auto t_bb = [&](int k, double(&acc)[1]) {
     if (rb + k * rs < n) acc[0] = fma(r[k], r[k], acc[0]);
   };
@@ -736,7 +794,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
       const int i = rb + k * rs;
       if (i < n) acc[0] = fma(__ldg(bg + i), v[k], acc[0]);
     };
-    if (!REF) {
+    if (!CHAIN) {
 #pragma unroll
       for (int k = 0; k < R; ++k) t_bv(k, q);
     }
@@ -753,7 +811,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
       if (i < n) {
         x[k] = fma(alpha, sph[i], x[k]);
         r[k] = fma(-alpha, v[k], r[k]);
-        if (!REF) q[0] = fma(r[k], r[k], q[0]);
+        if (!CHAIN) q[0] = fma(r[k], r[k], q[0]);
       }
     }
     BILU_RR_INPUT(r);
@@ -780,7 +838,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
         acc[1] = fma(t[k], t[k], acc[1]);
       }
     };
-    if (!REF) {
+    if (!CHAIN) {
 #pragma unroll
       for (int k = 0; k < R; ++k) t_ts(k, q2);
     }
@@ -804,7 +862,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
         x[k] = fma(omega, sph[i], x[k]);
         r[k] = fma(-omega, t[k], r[k]);
       }
-      if (!REF) t_rr(k, q2);
+      if (!CHAIN) t_rr(k, q2);
     }
     if (BILU_RR_SUM(2, q2, t_rr) && lane0) {
       bc[5] = sqrt(q2[0]);
@@ -823,7 +881,6 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     }
   }
 #undef BILU_RR_APPLY
-#undef BILU_RR_SUM
 #undef BILU_RR_INPUT
 
   // ---- write back
@@ -895,17 +952,17 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
 #pragma unroll
     for (int k = 0; k < R; ++k) {
       const int i = rb + k * rs;
-      if (i < n) {
-        const double ri = __ldg(bg + i) - ax[k];
-        q[0] = fma(ri, ri, q[0]);
-      }
+      r[k] = i < n ? __ldg(bg + i) - ax[k] : 0.0;
+      if (!CHAIN) t_bb(k, q);
     }
-    if (block_sum_w0<1, PV != 3>(q, red, nw) && tid == 0) a.true_res[sys] = sqrt(q[0]);
+    if (BILU_RR_SUM(1, q, t_bb) && lane0) a.true_res[sys] = sqrt(q[0]);
   }
 }
 
-// 8 rows per thread: 3 CTAs of 128 threads per SM
-#define BILU_RR_BOUNDS __launch_bounds__(R <= 1 ? 1024 : (R == 2 ? 512 : (R == 4 ? 256 : 128)), R == 8 ? 3 : 1)
+#undef BILU_RR_SUM
+
+// 5 to 8 rows per thread: 3 CTAs of 128 threads per SM
+#define BILU_RR_BOUNDS __launch_bounds__(R <= 1 ? 1024 : (R == 2 ? 512 : (R <= 4 ? 256 : 128)), R > 4 ? 3 : 1)
 
 }  // namespace
 }  // namespace bilu

@@ -23,25 +23,27 @@ __global__ void BILU_RR_BOUNDS k_bicgstab_rr_lu(const SolveArgs a, const RRLayou
 }
 
 template <typename FT, int ORD, int MC>
-const void* lu_r(int R) {
-  switch (R) {
+const void* lu_r(int slots) {
+  switch (slots) {
     case 1: return (const void*)k_bicgstab_rr_lu<1, FT, ORD, MC>;
     case 2: return (const void*)k_bicgstab_rr_lu<2, FT, ORD, MC>;
+    case 3: return (const void*)k_bicgstab_rr_lu<3, FT, ORD, MC>;
     case 4: return (const void*)k_bicgstab_rr_lu<4, FT, ORD, MC>;
+    case 6: return (const void*)k_bicgstab_rr_lu<6, FT, ORD, MC>;
     default: return (const void*)k_bicgstab_rr_lu<8, FT, ORD, MC>;
   }
 }
 
 template <int MC>
-const void* lu_mc(int fp32, int R, int ref) {
-  if (ref) return fp32 ? lu_r<float, kRef, MC>(R) : lu_r<double, kRef, MC>(R);
-  return fp32 ? lu_r<float, kFast, MC>(R) : lu_r<double, kFast, MC>(R);
+const void* lu_mc(int fp32, int slots, int ref) {
+  if (ref) return fp32 ? lu_r<float, kRef, MC>(slots) : lu_r<double, kRef, MC>(slots);
+  return fp32 ? lu_r<float, kFast, MC>(slots) : lu_r<double, kFast, MC>(slots);
 }
 
 }  // namespace
 
-const void* rr_lu_kernel(int fp32, int R, int ref, int mc) {
-  return mc == 2 ? lu_mc<2>(fp32, R, ref) : lu_mc<3>(fp32, R, ref);
+const void* rr_lu_kernel(int fp32, int slots, int ref, int mc) {
+  return mc == 2 ? lu_mc<2>(fp32, slots, ref) : lu_mc<3>(fp32, slots, ref);
 }
 
 }  // namespace bilu

@@ -10,20 +10,16 @@ namespace {
 // spilled values (tens of bytes per thread, through L1) and a smaller L1
 // beside the extra CTAs' shared memory.  Same arithmetic as k_bicgstab_rr at
 // the same threads per system:
-//   R = 8   128 threads, 4 CTAs per SM (128 registers instead of 168)
-//   R = 4   256 threads, 4 CTAs per SM (64 registers), 3 with ILU factors (85)
-//   R = 2   512 threads, 2 CTAs per SM (64 registers)
+//   R = 3, 4   256 threads, 4 CTAs per SM (64 registers), 3 with ILU factors (80)
+//   R = 2      512 threads, 2 CTAs per SM (64 registers)
 // FP64 issue bounds the solver, and its stalls are load and FP64 latency, so
 // more warps per SM keep the FP64 pipe busier.  Measured on GB300 with the
-// headline batch (4096 3D 10x10x10 systems, FP32 ISAI): 8 rows per thread on
-// 4 CTAs of 128 threads 4.23 ms per solve, 4 rows on 4 CTAs of 256 threads
-// 3.49 ms.  ILU factors at 8 rows per thread keep k_bicgstab_rr, whose
-// shared-memory layout admits 3 CTAs per SM anyway.  The plan's autotuner
-// chooses.
+// headline batch (4096 3D 10x10x10 systems, FP32 ISAI): 4 rows on 4 CTAs of 256
+// threads 3.37 ms per solve.  The plan's autotuner chooses.
 template <int R, int PV>
 struct OccBounds {
-  static constexpr int threads = R == 8 ? 128 : (R == 4 ? 256 : 512);
-  static constexpr int ctas = R == 8 ? 4 : (R == 4 ? (PV == 3 ? 3 : 4) : 2);
+  static constexpr int threads = R == 2 ? 512 : 256;
+  static constexpr int ctas = R == 2 ? 2 : (PV == 3 ? 3 : 4);
 };
 
 template <int R, int PV, typename FT>
@@ -38,21 +34,22 @@ __global__ void __launch_bounds__(OccBounds<R, PV>::threads, OccBounds<R, PV>::c
 }
 
 template <int PV, typename FT>
-const void* rr_occ_kernel_pv(int R) {
-  switch (R) {
+const void* rr_occ_kernel_pv(int slots) {
+  switch (slots) {
     case 2: return (const void*)k_bicgstab_rr_occ<2, PV, FT>;
+    case 3: return (const void*)k_bicgstab_rr_occ<3, PV, FT>;
     case 4: return (const void*)k_bicgstab_rr_occ<4, PV, FT>;
-    default: return PV == 3 ? nullptr : (const void*)k_bicgstab_rr_occ<(PV == 3 ? 4 : 8), PV, FT>;
+    default: return nullptr;
   }
 }
 
 }  // namespace
 
-const void* rr_occ_kernel(int pv, int fp32, int R) {
-  if (pv == 0) return rr_occ_kernel_pv<0, double>(R);
-  if (pv == 1) return fp32 ? rr_occ_kernel_pv<1, float>(R) : rr_occ_kernel_pv<1, double>(R);
-  if (pv == 2) return fp32 ? rr_occ_kernel_pv<2, float>(R) : rr_occ_kernel_pv<2, double>(R);
-  return fp32 ? rr_occ_kernel_pv<3, float>(R) : rr_occ_kernel_pv<3, double>(R);
+const void* rr_occ_kernel(int pv, int fp32, int slots) {
+  if (pv == 0) return rr_occ_kernel_pv<0, double>(slots);
+  if (pv == 1) return fp32 ? rr_occ_kernel_pv<1, float>(slots) : rr_occ_kernel_pv<1, double>(slots);
+  if (pv == 2) return fp32 ? rr_occ_kernel_pv<2, float>(slots) : rr_occ_kernel_pv<2, double>(slots);
+  return fp32 ? rr_occ_kernel_pv<3, float>(slots) : rr_occ_kernel_pv<3, double>(slots);
 }
 
 }  // namespace bilu
