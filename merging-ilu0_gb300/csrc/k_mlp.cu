@@ -25,6 +25,7 @@
 #include <cstdint>
 
 #include "bilu_internal.h"
+#include "k_intfp.cuh"
 #include "k_tc.cuh"
 
 namespace bilu {
@@ -64,19 +65,20 @@ __global__ void k_rowstats(const DevPattern P, int nsys, const double* __restric
   const int s = blockIdx.x;
   if (s >= nsys) return;
   // FP32 throughout (the features are FP32): FP64 division and square root
-  // are long instruction sequences on this part's FP64 pipe
+  // are long instruction sequences on this part's FP64 pipe, where hardware
+  // conversions run too (88 % of it at 4096 7x7x7 systems, 53 us)
   const double* As = A + (size_t)s * P.nnz;
   for (int i = threadIdx.x; i < P.n; i += blockDim.x) {
     const int b = P.rp[i], e = P.rp[i + 1], d = P.diag[i];
     float rn = 0.0f, cn = 0.0f, c = 0.0f;
     for (int k = b; k < e; ++k) {
-      const float a = (float)As[k];
+      const float a = ifp::f32(As[k]);
       rn = fmaf(a, a, rn);
       const int t = P.tpos[k];
       if (t >= 0) {
-        const float at = (float)As[t];
+        const float at = ifp::f32(As[t]);
         cn = fmaf(at, at, cn);
-        if (k < d) c = fmaf(a, at / (float)As[P.diag[P.ci[k]]], c);
+        if (k < d) c = fmaf(a, at / ifp::f32(As[P.diag[P.ci[k]]]), c);
       }
     }
     rown[(size_t)s * P.n + i] = sqrtf(rn);
@@ -100,7 +102,7 @@ __device__ __forceinline__ Feat features(const DevPattern& P, int s, int e, cons
   const int i = P.row_of[e], j = P.ci[e];
   const double* As = A + (size_t)s * P.nnz;
   const double aij = As[e];
-  const float fij = (float)aij, fii = (float)As[P.diag[i]], fjj = (float)As[P.diag[j]];
+  const float fij = ifp::f32(aij), fii = ifp::f32(As[P.diag[i]]), fjj = ifp::f32(As[P.diag[j]]);
   const float inv = 1.0f / (fii != 0.0f ? fabsf(fii) : 1.0f);
   const float ci_ = corr[(size_t)s * P.n + i], cj = corr[(size_t)s * P.n + j];
   r.f[0] = fij * inv;
