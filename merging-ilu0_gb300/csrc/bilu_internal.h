@@ -349,6 +349,10 @@ const void* rr_lu_kernel(int fp32, int slots, int ref, int mc);             // k
 const void* rr_occ_kernel(int pv, int fp32, int slots);                     // k_solve_rr_occ.cu
 cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int pv, int fp32, int ref, int occ,
                             int nsm, cudaStream_t st);
+// reference-order solver with the ISAI of L and U, several systems per CTA (k_solve_isai_ref.cu); maxa, maxi: the
+// longest rows of A and of aiL / aiU
+bool isai_ref_fits(int n, int fp32, int maxa, int maxi);
+cudaError_t launch_solve_isai_ref(const SolveArgs& a, int fp32, int maxa, int maxi, int nsm, cudaStream_t st);
 size_t solve_max_smem();
 cudaError_t launch_expand(const DevPattern& p, int nsys, const double* vin, double* vout, cudaStream_t st);
 cudaError_t launch_ilu0(const DevPattern& p, int nsys, const double* A, double* lu, int approach, int threads,

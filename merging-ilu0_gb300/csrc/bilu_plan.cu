@@ -1216,13 +1216,14 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
       }
     }
   }
-  int maxl = P->a_maxl;
+  int maxi = 0;  // longest row of aiL / aiU
   if (P->has_isai) {
     for (int i = 0; i < P->n; ++i) {
-      maxl = std::max(maxl, P->ail_rp[i + 1] - P->ail_rp[i]);
-      maxl = std::max(maxl, P->aiu_rp[i + 1] - P->aiu_rp[i]);
+      maxi = std::max(maxi, P->ail_rp[i + 1] - P->ail_rp[i]);
+      maxi = std::max(maxi, P->aiu_rp[i + 1] - P->aiu_rp[i]);
     }
   }
+  const int maxl = std::max(P->a_maxl, maxi);
   if (P->timing) cudaEventRecord(P->ev[1], st);
   if (sc.sell_u) {
     e = launch_to_sell(P->dp.su_src, P->dp.su_nnz, P->dp.aiu_nnz, nsys, a.aiu, ws + sc.usell, fp32 ? 4 : 8, st);
@@ -1234,7 +1235,12 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
     if (e != cudaSuccess) return cuda_err(e, "SELL copy of A");
     a.A_sell = (const double*)(ws + sc.asell);
   }
-  e = P->rr ? launch_solve_rr(a, P->rr_lay, P->rr_threads, P->rr_pv, fp32 ? 1 : 0,
+  // the reference's ISAI solvers: several systems per CTA, unless the caller asked for a CTA size
+  const bool isai_ref = !P->rr && a.prec == PK_ISAI && !P->general_isai && o.reduction != BILU_REDUCE_FAST &&
+                        o.threads_per_system == 0 && isai_ref_fits(P->n, fp32 ? 1 : 0, P->a_maxl, maxi);
+  e = isai_ref
+          ? launch_solve_isai_ref(a, fp32 ? 1 : 0, P->a_maxl, maxi, P->nsm, st)
+      : P->rr ? launch_solve_rr(a, P->rr_lay, P->rr_threads, P->rr_pv, fp32 ? 1 : 0,
                               o.reduction == BILU_REDUCE_FAST ? 0 : 1, P->rr_occ ? 1 : 0, P->nsm, st)
             : launch_solve(a, P->threads, fp32 ? 1 : 0, o.reduction == BILU_REDUCE_FAST ? 1 : 0, maxl, st);
   if (e != cudaSuccess) return cuda_err(e, "solver launch");
