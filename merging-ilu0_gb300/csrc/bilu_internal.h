@@ -118,6 +118,15 @@ struct DevPattern {
   const uint2* tc_lo = nullptr;
   const uint2* tc_up = nullptr;
   int tc_mc = 0;
+  // compact ILU(0) program, with the compact solve programs where the only
+  // dependency pairs are the diagonals' and nnz < 65535 (null: none).  Slot s of
+  // lower level l, at l * maxw_lo + s: ic_hdr.x = first factor position (bits
+  // 0-15; the lower entries, then the diagonal), lower entries (16-17), row
+  // (18-28), top bit of the third column (30), used (31); ic_hdr.y = the columns
+  // as in tc_*.  Entry j, at (3 l + j) * maxw_lo + s: position of its column's
+  // diagonal | position of the transposed entry << 16 (0xffff: none)
+  const uint2* ic_hdr = nullptr;
+  const unsigned* ic_ent = nullptr;
   // ILU(0) program of the register-resident solver's merged form (n <= 1024),
   // per lower level: header {off, w, len, 0}; slot s word j at prog[off + j*w + s]:
   // word 0 = number of op words that follow; ops per entry k of the row in
@@ -423,6 +432,7 @@ struct bilu_plan {
   std::vector<int> tp_lo_hdr, tp_lo, tp_up_hdr, tp_up;  // triangular-solve programs (DevPattern::tp_*)
   std::vector<int> tc_lo, tc_up;                         // compact solve programs (DevPattern::tc_*)
   int tc_mc = 0;
+  std::vector<int> ic_hdr, ic_ent;                       // compact ILU(0) program (DevPattern::ic_*)
   std::vector<int> ilu_hdr, ilu_prog;                    // ILU(0) program (DevPattern::ilu_*)
   std::vector<int> sa_off, sa_ci, sa_src, su_off, su_ci, su_src;  // SELL-32 layouts (DevPattern::sa_*, su_*)
   std::vector<int> pl_ent;  // ParILU entry classes (see DevPattern::pl_ent)

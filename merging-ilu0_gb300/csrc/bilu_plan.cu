@@ -267,8 +267,36 @@ void build_sell(int n, const std::vector<int>& rp, const std::vector<int>& ci, s
   }
 }
 
+// Compact ILU(0) program (DevPattern::ic_*).
+void build_compact_ilu(bilu_plan& P) {
+  P.ic_hdr.clear();
+  P.ic_ent.clear();
+  if (!P.tc_mc || P.nnz >= 65535) return;
+  for (int i = 0; i < P.n; ++i)
+    for (int k = P.rp[i]; k < P.rp[i + 1]; ++k)
+      if (k != P.diag[i] && P.dep_ptr[k + 1] > P.dep_ptr[k]) return;
+  const size_t W = P.maxw_lo, nlev = P.lev_lo_ptr.size() - 1;
+  P.ic_hdr.assign(2 * nlev * W, 0);
+  P.ic_ent.assign(3 * nlev * W, 0);
+  for (size_t l = 0; l < nlev; ++l)
+    for (int q = P.lev_lo_ptr[l]; q < P.lev_lo_ptr[l + 1]; ++q) {
+      const int i = P.lev_lo_rows[q], k0 = P.rp[i], cnt = P.diag[i] - k0;
+      const size_t s = q - P.lev_lo_ptr[l];
+      unsigned c[3] = {0, 0, 0};
+      for (int j = 0; j < cnt; ++j) {
+        c[j] = (unsigned)P.ci[k0 + j];
+        const int t = find_pos(P.rp, P.ci, P.ci[k0 + j], i);
+        P.ic_ent[(3 * l + j) * W + s] = (int)((unsigned)P.diag[c[j]] | (t < 0 ? 0xffffu : (unsigned)t) << 16);
+      }
+      P.ic_hdr[2 * (l * W + s)] =
+          (int)((unsigned)k0 | (unsigned)cnt << 16 | (unsigned)i << 18 | (c[2] >> 10) << 30 | 1u << 31);
+      P.ic_hdr[2 * (l * W + s) + 1] = (int)(c[0] | c[1] << 11 | c[2] << 22);
+    }
+}
+
 void build_deps(bilu_plan& P) {
   bilu::pattern_deps(P.n, P.rp.data(), P.ci.data(), P.diag.data(), P.dep_ptr, P.dep);
+  build_compact_ilu(P);
   P.ilu_hdr.clear();
   P.ilu_prog.clear();
   // the merged form's in-kernel ILU(0) in the register-resident solver (n <= 1024, 20-bit positions)
@@ -537,7 +565,7 @@ bilu_status upload(bilu_plan& P) {
   const size_t o_plent = put(P.pl_ent);
   const size_t o_plpp = put(P.pl_prog_ptr), o_plp = put(P.pl_prog);
   const size_t o_tlh = put(P.tp_lo_hdr), o_tl = put(P.tp_lo), o_tuh = put(P.tp_up_hdr), o_tu = put(P.tp_up);
-  const size_t o_tcl = put(P.tc_lo), o_tcu = put(P.tc_up);
+  const size_t o_tcl = put(P.tc_lo), o_tcu = put(P.tc_up), o_ich = put(P.ic_hdr), o_ice = put(P.ic_ent);
   const size_t o_sao = put(P.sa_off), o_sac = put(P.sa_ci), o_sas = put(P.sa_src);
   const size_t o_ih = put(P.ilu_hdr), o_ip = put(P.ilu_prog);
   // 16-bit column indices, two per int
@@ -686,6 +714,10 @@ bilu_status upload(bilu_plan& P) {
     d.tc_lo = reinterpret_cast<const uint2*>(b + o_tcl);
     d.tc_up = reinterpret_cast<const uint2*>(b + o_tcu);
     d.tc_mc = P.tc_mc;
+  }
+  if (!P.ic_hdr.empty()) {
+    d.ic_hdr = reinterpret_cast<const uint2*>(b + o_ich);
+    d.ic_ent = reinterpret_cast<const unsigned*>(b + o_ice);
   }
   d.pl_ndep = P.pl_ndep;
   d.pl_nlow = P.pl_nlow;

@@ -143,3 +143,78 @@ __device__ void ilu_program_rows(const DevPattern& P, double* LU, int approach, 
     for (int j = 0; j <= kIluPrefetch; ++j) w[j] = wn[j];
   }
 }
+
+// In-kernel ILU(0) from the plan's compact ILU program (DevPattern::ic_*; rows
+// of at most MC = 2 or 3 lower entries and dependency pairs on the diagonal
+// only, the 2D 5-point and 3D 7-point stencils): the same operations in the
+// same order as ilu_rows.  A row is l_k = a_ik / u_kk for its lower entries,
+// independent of each other, and the products l_k u_ki from the diagonal; its
+// words are loaded a level ahead.  The quotients come from the reciprocals of
+// the diagonals (ifp::quot, the value of the division), which the row that owns
+// the diagonal leaves in yinv (n doubles).  Block-wide; ends with a barrier.
+// Measured: see the kernels that use it (k_solve_rr_lu.cu, k_factor.cu).
+template <int MC>
+__device__ __forceinline__ void ilu_compact_rows(const DevPattern& P, double* LU, double* yinv, int approach, int tid,
+                                                 int nt) {
+  const int W = P.maxw_lo, nlev = P.nlev_lo;
+  const bool in_place = approach == 1 || approach == 4;
+  struct Row {
+    uint2 h;
+    unsigned e[MC];
+  };
+  auto fetch = [&](int lev, int s) {
+    Row r;
+    r.h = __ldg(P.ic_hdr + (size_t)lev * W + s);
+#pragma unroll
+    for (int j = 0; j < MC; ++j) r.e[j] = __ldg(P.ic_ent + ((size_t)lev * 3 + j) * W + s);
+    return r;
+  };
+  auto run = [&](const Row& r) {
+    if (!(r.h.x >> 31)) return;
+    const int k0 = r.h.x & 0xffff, cnt = (r.h.x >> 16) & 3, i = (r.h.x >> 18) & (kRRMaxRows - 1);
+    const int c[3] = {(int)(r.h.y & (kRRMaxRows - 1)), (int)((r.h.y >> 11) & (kRRMaxRows - 1)),
+                      (int)(r.h.y >> 22 | ((r.h.x >> 30) & 1) << 10)};
+    double l[MC], u[MC];
+    bool pair[MC];
+#pragma unroll
+    for (int j = 0; j < MC; ++j) {
+      l[j] = 0.0;
+      pair[j] = j < cnt && (r.e[j] >> 16) != 0xffffu;
+      u[j] = pair[j] ? LU[r.e[j] >> 16] : 0.0;
+      if (j < cnt) {
+        l[j] = ifp::quot(LU[k0 + j], LU[r.e[j] & 0xffff], yinv[c[j]]);
+        LU[k0 + j] = l[j];
+      }
+    }
+    double v = LU[k0 + cnt];
+    if (in_place) {
+#pragma unroll
+      for (int j = 0; j < MC; ++j)
+        if (pair[j]) v = fma(-l[j], u[j], v);
+    } else {
+      double s = 0.0;
+      if (approach == 3) {
+#pragma unroll
+        for (int j = 0; j < MC; ++j)
+          if (pair[j]) s = fma(l[j], u[j], s);
+      } else {
+#pragma unroll
+        for (int j = MC - 1; j >= 0; --j)
+          if (pair[j]) s = fma(l[j], u[j], s);
+      }
+      v = v - s;
+    }
+    LU[k0 + cnt] = v;
+    yinv[i] = ifp::quot_rcp(v);
+  };
+  Row cur;
+  if (tid < W) cur = fetch(0, tid);
+  for (int lev = 0; lev < nlev; ++lev) {
+    Row next = cur;
+    if (tid < W && lev + 1 < nlev) next = fetch(lev + 1, tid);
+    if (tid < W) run(cur);
+    for (int s = tid + nt; s < W; s += nt) run(fetch(lev, s));
+    __syncthreads();
+    cur = next;
+  }
+}

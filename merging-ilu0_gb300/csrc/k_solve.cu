@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include "bilu_internal.h"
+#include "k_intfp.cuh"
 
 namespace bilu {
 namespace {

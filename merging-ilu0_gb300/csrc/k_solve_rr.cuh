@@ -628,10 +628,17 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
       double* LUd = reinterpret_cast<double*>(smem + L.F);
       for (int k = tid; k < nnz; k += nt) LUd[k] = __ldg(Ag + k);
       __syncthreads();
-      if (P.ilu_prog && P.ilu_prog_approach == a.approach)
-        ilu_program_rows(P, LUd, a.approach, tid, nt);
-      else
-        ilu_rows(P, LUd, a.approach);
+      if constexpr (MC > 0) {
+        if (P.ic_hdr)
+          ilu_compact_rows<MC>(P, LUd, sph, a.approach, tid, nt);
+        else
+          ilu_rows(P, LUd, a.approach);
+      } else {
+        if (P.ilu_prog && P.ilu_prog_approach == a.approach)
+          ilu_program_rows(P, LUd, a.approach, tid, nt);
+        else
+          ilu_rows(P, LUd, a.approach);
+      }
       if (sizeof(FT) == 4) {
         // round to float in place, in chunks of 8 values per thread: chunk c's
         // float writes end at byte 4 * (its last index + 1), before the first
@@ -667,7 +674,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
           rinv[2 * n + i] = (FT)dgi;
         }
       } else {
-        rinv[i] = (FT)(1.0 / dgi);
+        rinv[i] = (FT)ifp::rcp(dgi);
       }
     }
     // visible to the solves after the first reduction's barrier

@@ -6,7 +6,8 @@
 // issue and the levels' latency.  Against the general programs: merged ILU(0)
 // of 4096 3D 10x10x10 systems, FAST order, 6.26 -> 5.43 ms; of 4096 2D 16x16
 // systems in the reference's order 3.08 -> 2.92 ms, of 8 2D 8x8 systems 276 ->
-// 224 us.
+// 224 us.  With the merged form's ILU(0) from its compact program too
+// (ilu_compact_rows) 5.45 -> 5.14 ms, 2.92 -> 2.78 ms, 224 -> 217 us.
 #include "k_solve_rr.cuh"
 
 namespace bilu {
