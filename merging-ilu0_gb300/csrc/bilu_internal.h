@@ -379,7 +379,7 @@ size_t mlp_train_smem();
 cudaError_t launch_mlp_train(const DevPattern& p, int nsys, const double* A, const double* LUt, const float* rown,
                              const float* coln, const float* corr, const void* pbf, int nsample, const int* idx,
                              uint64_t seed, float* grad, float* loss, cudaStream_t st);
-cudaError_t launch_mlp_adam(float* p, float* m, float* v, float* g, void* pbf, int count, float lr, int step,
+cudaError_t launch_mlp_adam(float* p, float* m, float* v, const float* g, void* pbf, int count, float lr, int step,
                             cudaStream_t st);
 cudaError_t launch_mlp_to_bf16(const float* p, void* pbf, int count, cudaStream_t st);
 cudaError_t launch_mlp_eval(const DevPattern& p, int nsys, const double* A, const float* rown, const float* coln,

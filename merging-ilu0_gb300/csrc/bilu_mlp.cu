@@ -163,8 +163,8 @@ bilu_status bilu_mlp_train(bilu_mlp* M, const bilu_plan* P, int nsys, const doub
   float* d_losses = nullptr;
   if (e == cudaSuccess && steps > 0) e = cudaMalloc((void**)&d_losses, steps * sizeof(float));
   if (e == cudaSuccess && steps > 0) e = cudaMemsetAsync(d_losses, 0, steps * sizeof(float), s);
-  if (e == cudaSuccess && steps > 0) e = cudaMemsetAsync(M->g, 0, kMlpParams * sizeof(float), s);  // k_adam zeroes it
   for (int t = 0; t < steps && e == cudaSuccess; ++t) {
+    e = cudaMemsetAsync(M->g, 0, kMlpParams * sizeof(float), s);
     if (e == cudaSuccess)
       e = launch_mlp_train(P->dp, nsys, d_values, d_lu_target, rown, coln, corr, M->pbf, batch, nullptr,
                            seed ^ (0xA24BAED4963EE407ull * (uint64_t)(M->step + 1)), M->g, d_losses + t, s);

@@ -179,14 +179,19 @@ __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bflo
   lo = __float2bfloat16_rn(x - __bfloat162float(hi));
 }
 
-// Sum over the 32 lanes of a warp of 16 values per lane, scattered: lanes l and
-// l + 16 return the warp's sum of v[l] (lane pairs 16 apart first, then
-// recursive halving).
-__device__ __forceinline__ float warp_reduce_scatter16(const float (&v)[16]) {
+// Sum over the 32 lanes of a warp of 32 values per lane, scattered: lane l
+// returns the warp's sum of v[l] (recursive halving, 31 shuffles).
+__device__ __forceinline__ float warp_reduce_scatter32(const float (&v)[32]) {
   const int lane = threadIdx.x & 31;
   float a[16];
+  {
+    const bool up = lane & 16;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) a[i] = v[i] + __shfl_xor_sync(kFull, v[i], 16);
+    for (int i = 0; i < 16; ++i) {
+      const float mine = up ? v[i + 16] : v[i], send = up ? v[i] : v[i + 16];
+      a[i] = mine + __shfl_xor_sync(kFull, send, 16);
+    }
+  }
 #pragma unroll
   for (int w = 8; w >= 1; w >>= 1) {
     const bool up = lane & w;
@@ -209,39 +214,30 @@ __device__ __forceinline__ float warp_reduce_scatter16(const float (&v)[16]) {
 //   BWV  [64] float2              (b2[u], w3[u])
 //   X    [128][9] FP32            features
 //   G1   [128][65] FP32           gelu'(pre1), later dpre1
-//   Y    [128] float2             target, 1 / 0 for samples that exist
-//   OUT  [128] FP32               the network's outputs
-//   RED  [3][4][64], [2][4] FP32  per-warp sums of db2, dW3, db1; of the loss and dout
-constexpr int TT = 512, TPARTS = TT / TB, TU = H / TPARTS;  // threads, threads per sample, units of each
+//   RED  [3][4][64] FP32          per-warp sums of db2, dW3, db1
 constexpr int TR_A1 = 0, TR_BT = TR_A1 + 2 * TB * H * 2, TR_AT = TR_BT + 2 * H * TB * 2, TR_BW = TR_AT + TB * TB * 2;
 constexpr int TR_BWT = TR_BW + H * H * 2, TR_W1 = TR_BWT + H * H * 2, TR_BWV = TR_W1 + H * 12 * 4;
-constexpr int TR_X = TR_BWV + H * 8, TR_G1 = TR_X + TB * NF * 4, TR_Y = TR_G1 + TB * LD * 4;
-constexpr int TR_OUT = TR_Y + TB * 8, TR_RED = TR_OUT + TB * 4, TR_SMEM = TR_RED + (12 * H + 8) * 4;
+constexpr int TR_X = TR_BWV + H * 8, TR_G1 = TR_X + TB * NF * 4, TR_RED = TR_G1 + TB * LD * 4;
+constexpr int TR_SMEM = TR_RED + 3 * 4 * H * 4;
 constexpr uint32_t kTrainTmemCols = 256;  // D1 pre2 | D2 dh1 | D3, D4 the two halves of dW2
-static_assert(TR_W1 % 16 == 0 && TR_X % 16 == 0 && TR_Y % 8 == 0 && TU == 16, "aligned blocks, one TMEM load a part");
+static_assert(TR_W1 % 16 == 0 && TR_X % 16 == 0, "aligned blocks");
 
-// One forward + backward pass over a block of 128 samples with the three
-// 64-wide GEMMs on the tensor cores (tcgen05.mma, BF16 operands split into high
-// and low parts, FP32 accumulators in TMEM):
+// One forward + backward pass over a block of 128 samples (thread = sample) with
+// the three 64-wide GEMMs on the tensor cores (tcgen05.mma, BF16 operands
+// split into high and low parts, FP32 accumulators in TMEM):
 //   forward   pre2 = H1 W2^T                 (M = 128 samples, N = 64, K = 64)
 //   backward  dh1  = dpre2 W2                (M = 128 samples, N = 64, K = 64)
 //             dW2  = dpre2^T H1              (M = 128: the 64 units' high and low
 //                                             parts stacked, N = 64, K = 128 samples)
 // Layer 1, the activations and the output layer run on the CUDA cores in FP32
-// with the accurate tanh.  What bounds it is the latency of those steps between
-// the GEMMs on the one CTA that 159 KB of shared memory let an SM hold, so a
-// sample is four threads (16 units each: warp w has the samples of TMEM lanes
-// 32 (w % 4) .. + 31 and the units 16 (w / 4) .. + 15): a step of 65536 samples
-// 187 -> 86 us.  Every block adds the sums of one thread per sample to `grad`
-// (FP32 atomics; their rounding too, the order of units and samples being that
-// of one thread per sample).  Persistent CTAs that add up four blocks first take
-// 64 us, but the losses, which magnify a BF16 rounding of a weight that falls
-// the other way, then move by more than they do from run to run.
-// The summed squared error goes to `loss`.  Samples: explicit global entry
-// indices (s*nnz+e) or, when idx == NULL, hashed from (seed, sample number).  A
-// tensor-core round that does not complete within the bounded wait adds NaN to
-// `loss` and ends the block.
-__global__ void __launch_bounds__(TT) k_mlp_train(const DevPattern P, int nsys, const double* __restrict__ A,
+// with the accurate tanh.  Per-unit sums over the block (db1, db2, dW3) are
+// reduce-scattered across each warp; dW1 is reduced over the block in shared
+// memory; everything is added to `grad` (FP32 atomics), the summed squared
+// error to `loss`.  Samples: explicit global entry indices (s*nnz+e) or, when
+// idx == NULL, hashed from (seed, sample number).  A tensor-core round that
+// does not complete within the bounded wait adds NaN to `loss` and ends the
+// block.
+__global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, const double* __restrict__ A,
                                                   const double* __restrict__ LUt, const float* __restrict__ rown,
                                                   const float* __restrict__ coln, const float* __restrict__ corr,
                                                   const __nv_bfloat16* __restrict__ pbf, int nsample,
@@ -250,34 +246,32 @@ __global__ void __launch_bounds__(TT) k_mlp_train(const DevPattern P, int nsys, 
   extern __shared__ __align__(1024) unsigned char smt[];
   __shared__ uint64_t s_mbar;
   __shared__ uint32_t s_tmem;
+  __shared__ float s_loss[TB / 32], s_do[TB / 32];
   __shared__ int s_fail;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t = tid & (TB - 1), part = tid >> 7;  // sample of the block, which 16 units
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   float* X = reinterpret_cast<float*>(smt + TR_X);
   float* G1 = reinterpret_cast<float*>(smt + TR_G1);
-  float2* Y = reinterpret_cast<float2*>(smt + TR_Y);
   float* RED = reinterpret_cast<float*>(smt + TR_RED);
-  float* OUT = reinterpret_cast<float*>(smt + TR_OUT);
   // ---- weights
   {
     const uint4* w2g = reinterpret_cast<const uint4*>(pbf + OW2);
-    for (int k = tid; k < H * 8; k += TT) {
+    for (int k = t; k < H * 8; k += TB) {
       const int u = k >> 3, c = k & 7;
       *reinterpret_cast<uint4*>(smt + TR_BW + tc::kmajor_off(u, 8 * c, H)) = w2g[k];
     }
-    for (int k = tid; k < H * H; k += TT) {  // W2^T: element (v, u) = W2[u][v]
+    for (int k = t; k < H * H; k += TB) {  // W2^T: element (v, u) = W2[u][v]
       const int u = k >> 6, v = k & 63;
       *reinterpret_cast<__nv_bfloat16*>(smt + TR_BWT + tc::kmajor_off(v, u, H)) = pbf[OW2 + k];
     }
     float* w1 = reinterpret_cast<float*>(smt + TR_W1);
-    for (int k = tid; k < H * 12; k += TT) {
+    for (int k = t; k < H * 12; k += TB) {
       const int v = k / 12, c = k % 12;
       w1[k] = c < NF ? __bfloat162float(pbf[OW1 + v * NF + c]) : (c == NF ? __bfloat162float(pbf[OB1 + v]) : 0.0f);
     }
     float2* bwv = reinterpret_cast<float2*>(smt + TR_BWV);
-    for (int u = tid; u < H; u += TT) bwv[u] = make_float2(__bfloat162float(pbf[OB2 + u]), __bfloat162float(pbf[OW3 + u]));
+    for (int u = t; u < H; u += TB) bwv[u] = make_float2(__bfloat162float(pbf[OB2 + u]), __bfloat162float(pbf[OW3 + u]));
   }
-  if (tid == 0) {
+  if (t == 0) {
     tc::mbar_init(&s_mbar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_fail = 0;
@@ -287,149 +281,141 @@ __global__ void __launch_bounds__(TT) k_mlp_train(const DevPattern P, int nsys, 
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = s_tmem;
-  const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+  const uint32_t trow = tmem + ((uint32_t)(32 * warp) << 16);
   const float4* w1v = reinterpret_cast<const float4*>(smt + TR_W1);
-  const float2* bwv = reinterpret_cast<const float2*>(smt + TR_BWV) + TU * part;
+  const float2* bwv = reinterpret_cast<const float2*>(smt + TR_BWV);
   const float b3 = __bfloat162float(pbf[OB3]);
+  // ---- sample, features, target
+  const long long q = (long long)blockIdx.x * TB + t;
+  const bool live = q < nsample;
+  float f[NF];
+  float ytrue = 0.0f;
+  if (live) {
+    long long g;
+    if (idx) {
+      g = idx[q];
+    } else {  // a random system and a random entry among those the network predicts
+      const uint64_t h = mix64(seed ^ (0x9E3779B97F4A7C15ull * (uint64_t)(q + 1)));
+      g = (long long)(h % (uint64_t)nsys) * P.nnz + P.mlp_ent[(h >> 32) % (uint64_t)P.n_mlp];
+    }
+    const int s = (int)(g / P.nnz), e = (int)(g % P.nnz);
+    const Feat ft = features(P, s, e, A, rown, coln, corr);
+#pragma unroll
+    for (int k = 0; k < NF; ++k) f[k] = ft.f[k];
+    const double denom = ft.a * (double)ft.base;
+    ytrue = denom != 0.0 ? (float)(LUt[g] / denom - 1.0) : 0.0f;
+  } else {
+#pragma unroll
+    for (int k = 0; k < NF; ++k) f[k] = 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < NF; ++k) X[t * NF + k] = live ? f[k] : 0.0f;
+  // ---- layer 1 (CUDA cores): H1 hi / lo into A1 (row t) and BT (column t), gelu'(pre1) into G1
   __nv_bfloat16* bth = reinterpret_cast<__nv_bfloat16*>(smt + TR_BT);
   __nv_bfloat16* btl = reinterpret_cast<__nv_bfloat16*>(smt + TR_BT + H * TB * 2);
-  __nv_bfloat16* ath = reinterpret_cast<__nv_bfloat16*>(smt + TR_AT);
+#pragma unroll 1
+  for (int c = 0; c < H / 8; ++c) {
+    __align__(16) __nv_bfloat16 hi[8], lo[8];
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+      const int v = 8 * c + d;
+      const float4 wa = w1v[v * 3], wb = w1v[v * 3 + 1], wc = w1v[v * 3 + 2];
+      const float w[NF] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w, wc.x};
+      float pre = wc.y;
+#pragma unroll
+      for (int k = 0; k < NF; ++k) pre = fmaf(w[k], f[k], pre);
+      const float h = live ? gelu(pre) : 0.0f;
+      G1[t * LD + v] = live ? gelu_d(pre) : 0.0f;
+      split_bf16(h, hi[d], lo[d]);
+      const uint32_t bo = tc::kmajor_off(v, t, TB) / 2;
+      bth[bo] = hi[d];
+      btl[bo] = lo[d];
+    }
+    const uint32_t off = tc::kmajor_off(t, 8 * c, H);
+    *reinterpret_cast<uint4*>(smt + TR_A1 + off) = *reinterpret_cast<const uint4*>(hi);
+    *reinterpret_cast<uint4*>(smt + TR_A1 + TB * H * 2 + off) = *reinterpret_cast<const uint4*>(lo);
+  }
   const uint32_t a1h = tc::smem_u32(smt + TR_A1), a1l = a1h + TB * H * 2;
   const uint32_t bth_a = tc::smem_u32(smt + TR_BT), btl_a = bth_a + H * TB * 2;
   const uint32_t at_a = tc::smem_u32(smt + TR_AT), bw_a = tc::smem_u32(smt + TR_BW), bwt_a = tc::smem_u32(smt + TR_BWT);
   constexpr uint32_t kSbo64 = H * 16, kSbo128 = TB * 16;
   const uint32_t id128 = tc::idesc_bf16(128, H);
-  uint32_t phase = 0;
-  // waits (bounded) for the MMAs committed last; false (uniformly) when they did not complete
-  auto round_done = [&]() {
-    if (!tc::mbar_wait(&s_mbar, phase, kWaitLimit)) s_fail = 1;
-    phase ^= 1u;
-    tc::fence_after_sync();
-    __syncthreads();
-    return s_fail == 0;
-  };
-  // row t's units u .. u + 7 of a K-major operand pair (hi, lo): one 16-byte chunk each
-  auto store_row = [&](int u, const __nv_bfloat16 (&hi)[8], const __nv_bfloat16 (&lo)[8]) {
-    const uint32_t off = tc::kmajor_off(t, u, H);
-    *reinterpret_cast<uint4*>(smt + TR_A1 + off) = *reinterpret_cast<const uint4*>(hi);
-    *reinterpret_cast<uint4*>(smt + TR_A1 + TB * H * 2 + off) = *reinterpret_cast<const uint4*>(lo);
-  };
-
-  // ---- sample, features, target
-  if (part == 0) {
-    const long long q = (long long)blockIdx.x * TB + t;
-    float f[NF] = {}, ytrue = 0.0f, live = 0.0f;
-    if (q < nsample) {
-      long long g;
-      if (idx) {
-        g = idx[q];
-      } else {  // a random system and a random entry among those the network predicts
-        const uint64_t h = mix64(seed ^ (0x9E3779B97F4A7C15ull * (uint64_t)(q + 1)));
-        g = (long long)(h % (uint64_t)nsys) * P.nnz + P.mlp_ent[(h >> 32) % (uint64_t)P.n_mlp];
-      }
-      const int s = (int)(g / P.nnz), e = (int)(g % P.nnz);
-      const Feat ft = features(P, s, e, A, rown, coln, corr);
-#pragma unroll
-      for (int k = 0; k < NF; ++k) f[k] = ft.f[k];
-      const double denom = ft.a * (double)ft.base;
-      ytrue = denom != 0.0 ? (float)(LUt[g] / denom - 1.0) : 0.0f;
-      live = 1.0f;
-    }
-#pragma unroll
-    for (int k = 0; k < NF; ++k) X[t * NF + k] = f[k];
-    Y[t] = make_float2(ytrue, live);
-  }
+  // ---- forward layer 2 on the tensor cores: D1 = H1 W2^T
+  tc::fence_smem_to_async();
+  tc::fence_before_sync();
   __syncthreads();
-  do {
-    const float2 yl = Y[t];
-    // ---- layer 1 (CUDA cores): H1 hi / lo into A1 (row t) and BT (column t), gelu'(pre1) into G1
-    {
-      float x[NF];
+  if (t == 0) {
+    tc::fence_after_sync();
 #pragma unroll
-      for (int k = 0; k < NF; ++k) x[k] = X[t * NF + k];
-#pragma unroll 1
-      for (int c = 0; c < TU; c += 8) {
-        __align__(16) __nv_bfloat16 hi[8], lo[8];
+    for (int j = 0; j < H / 16; ++j)
+      tc::mma_bf16(tmem, tc::sdesc(a1h + 256 * j, kSbo64), tc::sdesc(bw_a + 256 * j, kSbo64), id128, j > 0);
 #pragma unroll
-        for (int d = 0; d < 8; ++d) {
-          const int v = TU * part + c + d;
-          const float4 wa = w1v[v * 3], wb = w1v[v * 3 + 1], wc = w1v[v * 3 + 2];
-          const float w[NF] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w, wc.x};
-          float pre = wc.y;
-#pragma unroll
-          for (int k = 0; k < NF; ++k) pre = fmaf(w[k], x[k], pre);
-          const float h = yl.y != 0.0f ? gelu(pre) : 0.0f;
-          G1[t * LD + v] = yl.y != 0.0f ? gelu_d(pre) : 0.0f;
-          split_bf16(h, hi[d], lo[d]);
-          const uint32_t bo = tc::kmajor_off(v, t, TB) / 2;
-          bth[bo] = hi[d];
-          btl[bo] = lo[d];
-        }
-        store_row(TU * part + c, hi, lo);
-      }
-    }
-    // ---- forward layer 2 on the tensor cores: D1 = H1 W2^T
-    tc::fence_smem_to_async();
-    tc::fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc::fence_after_sync();
-#pragma unroll
-      for (int j = 0; j < H / 16; ++j)
-        tc::mma_bf16(tmem, tc::sdesc(a1h + 256 * j, kSbo64), tc::sdesc(bw_a + 256 * j, kSbo64), id128, j > 0);
-#pragma unroll
-      for (int j = 0; j < H / 16; ++j)
-        tc::mma_bf16(tmem, tc::sdesc(a1l + 256 * j, kSbo64), tc::sdesc(bw_a + 256 * j, kSbo64), id128, 1);
-      tc::commit(&s_mbar);
-    }
-    if (!round_done()) break;
+    for (int j = 0; j < H / 16; ++j)
+      tc::mma_bf16(tmem, tc::sdesc(a1l + 256 * j, kSbo64), tc::sdesc(bw_a + 256 * j, kSbo64), id128, 1);
+    tc::commit(&s_mbar);
+  }
+  if (!tc::mbar_wait(&s_mbar, 0, kWaitLimit)) s_fail = 1;  // 1 + the parity of the phase that did not complete
+  tc::fence_after_sync();
+  __syncthreads();
+  if (s_fail) {
+    if (t == 0) atomicAdd(loss, __int_as_float(0x7fc00000));
+  } else {
     // ---- output layer, loss, dout
-    float pre2[TU], g2[TU];
-    tc::ld16(trow + TU * part, pre2);
+    float out = b3;
+#pragma unroll 1
+    for (int c = 0; c < H / 16; ++c) {
+      float acc[16];
+      tc::ld16(trow + 16 * c, acc);
 #pragma unroll
-    for (int k = 0; k < TU; ++k) {
-      pre2[k] += bwv[k].x;
-      g2[k] = gelu(pre2[k]);
-    }
-    // the output is one chain over the units, part after part: its rounding is that of one thread per sample
-    // (a loss far below the outputs' size shows a change of it)
-#pragma unroll
-    for (int p = 0; p < TPARTS; ++p) {
-      if (part == p) {
-        float out = p == 0 ? b3 : OUT[t];
-#pragma unroll
-        for (int k = 0; k < TU; ++k) out = fmaf(bwv[k].y, g2[k], out);
-        OUT[t] = out;
+      for (int k = 0; k < 16; ++k) {
+        const float2 bw = bwv[16 * c + k];
+        out = fmaf(bw.y, gelu(acc[k] + bw.x), out);
       }
-      __syncthreads();
     }
-    const float out = OUT[t];
-    const float diff = out - yl.x;
-    const float dout = yl.y != 0.0f ? 2.0f * diff * scale : 0.0f;
-    float l = yl.y != 0.0f ? diff * diff : 0.0f, dsum = dout;
-    // ---- dpre2 = dout w3 gelu'(pre2) into A1 (row t) and AT (column t); per-unit sums of dpre2 (db2) and of
-    // dout gelu(pre2) (dW3), reduce-scattered over the warp
-    {
+    const float diff = out - ytrue;
+    const float err2 = live ? diff * diff : 0.0f;
+    const float dout = live ? 2.0f * diff * scale : 0.0f;
+    // ---- dpre2 = dout w3 gelu'(pre2) into A1 (row t) and AT (column t); per-unit sums of dpre2 (db2)
+    // and of dout gelu(pre2) (dW3), reduce-scattered over the warp: lane l holds units l and 32 + l
+    __nv_bfloat16* ath = reinterpret_cast<__nv_bfloat16*>(smt + TR_AT);
+    float rs_db2[2], rs_dw3[2];
+#pragma unroll 1
+    for (int c2 = 0; c2 < 2; ++c2) {
+      float dp[32], dw[32];
 #pragma unroll
-      for (int c = 0; c < TU; c += 8) {
+      for (int h16 = 0; h16 < 2; ++h16) {
+        float acc[16];
+        tc::ld16(trow + 32 * c2 + 16 * h16, acc);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const int u = 32 * c2 + 16 * h16 + k;
+          const float pre = acc[k] + bwv[u].x;
+          dp[16 * h16 + k] = dout * bwv[u].y * gelu_d(pre);
+          dw[16 * h16 + k] = dout * gelu(pre);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
         __align__(16) __nv_bfloat16 hi[8], lo[8];
 #pragma unroll
         for (int d = 0; d < 8; ++d) {
-          const int k = c + d, u = TU * part + k;
-          pre2[k] = dout * bwv[k].y * gelu_d(pre2[k]);
-          g2[k] = dout * g2[k];
-          split_bf16(pre2[k], hi[d], lo[d]);
+          const int u = 32 * c2 + 8 * c + d;
+          split_bf16(dp[8 * c + d], hi[d], lo[d]);
           ath[tc::kmajor_off(u, t, TB) / 2] = hi[d];
           ath[tc::kmajor_off(H + u, t, TB) / 2] = lo[d];
         }
-        store_row(TU * part + c, hi, lo);
+        const uint32_t off = tc::kmajor_off(t, 32 * c2 + 8 * c, H);
+        *reinterpret_cast<uint4*>(smt + TR_A1 + off) = *reinterpret_cast<const uint4*>(hi);
+        *reinterpret_cast<uint4*>(smt + TR_A1 + TB * H * 2 + off) = *reinterpret_cast<const uint4*>(lo);
       }
+      rs_db2[c2] = warp_reduce_scatter32(dp);
+      rs_dw3[c2] = warp_reduce_scatter32(dw);
     }
     // ---- backward GEMMs on the tensor cores: D2 = dpre2 W2, D3 / D4 = dpre2^T (hi | lo stacked) H1 (hi / lo)
     tc::fence_smem_to_async();
     tc::fence_before_sync();
     __syncthreads();
-    if (tid == 0) {
+    if (t == 0) {
       tc::fence_after_sync();
 #pragma unroll
       for (int j = 0; j < H / 16; ++j)
@@ -447,83 +433,104 @@ __global__ void __launch_bounds__(TT) k_mlp_train(const DevPattern P, int nsys, 
                      j > 0);
       tc::commit(&s_mbar);
     }
-    // per-unit sums of the warps, the loss and the sum of dout (db3) while the tensor cores run
-    const float r_db2 = warp_reduce_scatter16(pre2), r_dw3 = warp_reduce_scatter16(g2);
-    const int w4 = warp & 3;
-    if (lane < TU) {
-      RED[(0 * 4 + w4) * H + TU * part + lane] = r_db2;
-      RED[(1 * 4 + w4) * H + TU * part + lane] = r_dw3;
-    }
-    if (part == 0) {
+    // loss and the sum of dout (db3) while the tensor cores run
+    float l = err2, dsum = dout;
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        l += __shfl_down_sync(kFull, l, off);
-        dsum += __shfl_down_sync(kFull, dsum, off);
-      }
-      if (lane == 0) {
-        RED[12 * H + w4] = l;
-        RED[12 * H + 4 + w4] = dsum;
-      }
+    for (int off = 16; off > 0; off >>= 1) {
+      l += __shfl_down_sync(kFull, l, off);
+      dsum += __shfl_down_sync(kFull, dsum, off);
     }
-    if (!round_done()) break;
-    // ---- dpre1 = dh1 * gelu'(pre1) into G1; per-unit sums of dpre1 (db1)
-    {
-      float d1[TU], d4[TU];
-      tc::ld16(trow + 64 + TU * part, d1);
-#pragma unroll
-      for (int k = 0; k < TU; ++k) {
-        float* g = G1 + t * LD + TU * part + k;
-        d1[k] *= *g;
-        *g = d1[k];
-      }
-      const float r_db1 = warp_reduce_scatter16(d1);
-      if (lane < TU) RED[(2 * 4 + w4) * H + TU * part + lane] = r_db1;
-      // ---- dW2: row r of D3 + D4 is unit r % 64's share (high part for r < 64, low part above)
-      tc::ld16(trow + 128 + TU * part, d1);
-      tc::ld16(trow + 192 + TU * part, d4);
-      float* g = grad + OW2 + (t & (H - 1)) * H + TU * part;
-#pragma unroll
-      for (int k = 0; k < TU; k += 4)
-        atomicAdd(reinterpret_cast<float4*>(g + k), make_float4(d1[k] + d4[k], d1[k + 1] + d4[k + 1],
-                                                                d1[k + 2] + d4[k + 2], d1[k + 3] + d4[k + 3]));
+    if (lane == 0) {
+      s_loss[warp] = l;
+      s_do[warp] = dsum;
     }
+    RED[(0 * 4 + warp) * H + lane] = rs_db2[0];
+    RED[(0 * 4 + warp) * H + 32 + lane] = rs_db2[1];
+    RED[(1 * 4 + warp) * H + lane] = rs_dw3[0];
+    RED[(1 * 4 + warp) * H + 32 + lane] = rs_dw3[1];
+    if (!tc::mbar_wait(&s_mbar, 1, kWaitLimit)) s_fail = 2;
+    tc::fence_after_sync();
     __syncthreads();
-    if (tid < 3 * H) {
-      const float* r = RED + (tid / H) * 4 * H + tid % H;
-      const int o = tid < H ? OB2 : (tid < 2 * H ? OW3 : OB1);
-      atomicAdd(grad + o + tid % H, ((r[0] + r[H]) + r[2 * H]) + r[3 * H]);
-    } else if (tid < 3 * H + 2) {
-      const float* r = RED + 12 * H + 4 * (tid - 3 * H);
-      const float v = ((r[0] + r[1]) + r[2]) + r[3];
-      atomicAdd(tid == 3 * H ? loss : grad + OB3, tid == 3 * H ? v * scale : v);
+    if (s_fail) {
+      if (t == 0) atomicAdd(loss, __int_as_float(0x7fc00000));
+    } else {
+      // ---- dpre1 = dh1 * gelu'(pre1) into G1; per-unit sums of dpre1 (db1)
+      float rs_db1[2];
+#pragma unroll 1
+      for (int c2 = 0; c2 < 2; ++c2) {
+        float dp[32];
+#pragma unroll
+        for (int h16 = 0; h16 < 2; ++h16) {
+          float acc[16];
+          tc::ld16(trow + 64 + 32 * c2 + 16 * h16, acc);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const int v = 32 * c2 + 16 * h16 + k;
+            const float d = acc[k] * G1[t * LD + v];
+            G1[t * LD + v] = d;
+            dp[16 * h16 + k] = d;
+          }
+        }
+        rs_db1[c2] = warp_reduce_scatter32(dp);
+      }
+      RED[(2 * 4 + warp) * H + lane] = rs_db1[0];
+      RED[(2 * 4 + warp) * H + 32 + lane] = rs_db1[1];
+      // ---- dW2: row r of D3 + D4 is unit r % 64's share (high part for r < 64, low part above)
+      {
+        const int u = (32 * warp + lane) & 63;
+#pragma unroll 1
+        for (int c = 0; c < H / 16; ++c) {
+          float d3[16], d4[16];
+          tc::ld16(trow + 128 + 16 * c, d3);
+          tc::ld16(trow + 192 + 16 * c, d4);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) atomicAdd(grad + OW2 + u * H + 16 * c + k, d3[k] + d4[k]);
+        }
+      }
+      __syncthreads();
+      if (t == 0) {
+        float a = 0.0f, d = 0.0f;
+        for (int w = 0; w < TB / 32; ++w) {
+          a += s_loss[w];
+          d += s_do[w];
+        }
+        atomicAdd(loss, a * scale);
+        atomicAdd(grad + OB3, d);
+      }
+      if (t < H) {
+        float db2 = 0.0f, dw3 = 0.0f, db1 = 0.0f;
+        for (int w = 0; w < TB / 32; ++w) {
+          db2 += RED[(0 * 4 + w) * H + t];
+          dw3 += RED[(1 * 4 + w) * H + t];
+          db1 += RED[(2 * 4 + w) * H + t];
+        }
+        atomicAdd(grad + OB2 + t, db2);
+        atomicAdd(grad + OW3 + t, dw3);
+        atomicAdd(grad + OB1 + t, db1);
+      }
+      for (int k = t; k < H * NF; k += TB) {  // dW1[u][f] = sum_t dpre1[t][u] * x[t][f]
+        const int u = k / NF, fi = k % NF;
+        float acc = 0.0f;
+        for (int r = 0; r < TB; ++r) acc = fmaf(G1[r * LD + u], X[r * NF + fi], acc);
+        atomicAdd(grad + OW1 + k, acc);
+      }
     }
-    for (int k = TT - 1 - tid; k < H * NF; k += TT) {  // dW1[u][f] = sum_t dpre1[t][u] * x[t][f]
-      const int u = k / NF, fi = k % NF;
-      float acc = 0.0f;
-#pragma unroll 16
-      for (int r = 0; r < TB; ++r) acc = fmaf(G1[r * LD + u], X[r * NF + fi], acc);
-      atomicAdd(grad + OW1 + k, acc);
-    }
-  } while (false);
-  if (s_fail) {
-    if (tid == 0) atomicAdd(loss, __int_as_float(0x7fc00000));
-    // the round that timed out may still be in flight: wait once more (bounded) before freeing its columns
-    tc::mbar_wait(&s_mbar, phase ^ 1u, kWaitLimit);
   }
+  // a round that timed out may still be in flight: wait once more (bounded) before freeing its columns
+  if (s_fail) tc::mbar_wait(&s_mbar, (uint32_t)(s_fail - 1), kWaitLimit);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   if (warp == 0) tc::dealloc(tmem, kTrainTmemCols);
 }
 
-// Adam on the FP32 master parameters; refreshes the BF16 copy and zeroes the
-// gradient for the next step's sums.
-__global__ void k_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float* __restrict__ g, __nv_bfloat16* __restrict__ pbf, int count, float lr, float b1,
+// Adam on the FP32 master parameters; refreshes the BF16 copy.
+__global__ void k_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
+                       const float* __restrict__ g, __nv_bfloat16* __restrict__ pbf, int count, float lr, float b1,
                        float b2, float eps, float c1, float c2) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= count) return;
   const float gk = g[k];
-  g[k] = 0.0f;
   const float mk = b1 * m[k] + (1.0f - b1) * gk;
   const float vk = b2 * v[k] + (1.0f - b2) * gk * gk;
   m[k] = mk;
@@ -837,12 +844,13 @@ cudaError_t launch_mlp_train(const DevPattern& p, int nsys, const double* A, con
   const size_t smem = mlp_train_smem();
   cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_mlp_train<<<(nsample + TB - 1) / TB, TT, smem, st>>>(p, nsys, A, LUt, rown, coln, corr, (const __nv_bfloat16*)pbf,
-                                                         nsample, idx, seed, 1.0f / (float)nsample, grad, loss);
+  k_mlp_train<<<(nsample + TB - 1) / TB, TB, smem, st>>>(p, nsys, A, LUt, rown, coln, corr,
+                                                         (const __nv_bfloat16*)pbf, nsample, idx, seed,
+                                                         1.0f / (float)nsample, grad, loss);
   return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_adam(float* p, float* m, float* v, float* g, void* pbf, int count, float lr, int step,
+cudaError_t launch_mlp_adam(float* p, float* m, float* v, const float* g, void* pbf, int count, float lr, int step,
                             cudaStream_t st) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
