@@ -674,7 +674,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
           rinv[2 * n + i] = (FT)dgi;
         }
       } else {
-        rinv[i] = (FT)ifp::rcp(dgi);
+        rinv[i] = (FT)(1.0 / dgi);
       }
     }
     // visible to the solves after the first reduction's barrier
