@@ -1,8 +1,9 @@
 // Device code of the register-resident batched BiCGSTAB solver, shared by
 // the translation units that instantiate its kernels (k_solve_rr.cu: the
-// main kernel and the launch code; k_solve_rr_occ.cu: the occupancy
-// variants; k_solve_rr_uneven.cu: the uneven-batch kernel), which compile
-// in parallel.  Everything here is in an anonymous namespace: each unit
+// main kernel and the launch code; k_solve_rr_occ.cu: the occupancy variants;
+// k_solve_rr_split.cu: several threads per order thread; k_solve_rr_lu.cu: ILU
+// factors of stencils; k_solve_rr_wide.cu: 1025 to 2048 rows;
+// k_solve_rr_uneven.cu: the uneven-batch kernel), which compile in parallel.  Everything here is in an anonymous namespace: each unit
 // gets its own copy of what it instantiates.
 //
 // Register-resident batched BiCGSTAB for BILU_REDUCE_FAST with an ISAI
