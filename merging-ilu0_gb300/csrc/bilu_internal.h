@@ -376,9 +376,12 @@ cudaError_t launch_dense_solve(const DevPattern& p, int nsample, const int* sys_
 cudaError_t launch_mlp_rowstats(const DevPattern& p, int nsys, const double* A, float* rown, float* coln, float* corr,
                                 cudaStream_t st);
 size_t mlp_train_smem();
+// loss and gradient of a batch (overwritten); work: mlp_train_work(nrows) bytes for at most nrows blocks at a time
+int mlp_train_rows(int nsample, int nsm);
+size_t mlp_train_work(int nrows);
 cudaError_t launch_mlp_train(const DevPattern& p, int nsys, const double* A, const double* LUt, const float* rown,
                              const float* coln, const float* corr, const void* pbf, int nsample, const int* idx,
-                             uint64_t seed, float* grad, float* loss, cudaStream_t st);
+                             uint64_t seed, float* work, int nrows, float* grad, float* loss, cudaStream_t st);
 cudaError_t launch_mlp_adam(float* p, float* m, float* v, const float* g, void* pbf, int count, float lr, int step,
                             cudaStream_t st);
 cudaError_t launch_mlp_to_bf16(const float* p, void* pbf, int count, cudaStream_t st);

@@ -19,14 +19,15 @@ struct bilu_mlp {
   float* p = nullptr;   // FP32 master parameters
   float* m = nullptr;   // Adam moments
   float* v = nullptr;
-  float* g = nullptr;   // gradient accumulator
+  float* g = nullptr;   // gradient
   void* pbf = nullptr;  // BF16 compute copy
-  float* loss = nullptr;
   int step = 0;
   float* stats = nullptr;  // row statistics scratch (3 * nsys * n floats)
   size_t stats_cap = 0;
   int* idx = nullptr;      // sample-index scratch
   size_t idx_cap = 0;
+  float* work = nullptr;   // gradient parts of a batch's blocks, then the losses of a call's steps
+  size_t work_cap = 0;     // bytes
 };
 
 namespace {
@@ -69,6 +70,25 @@ bilu_status ensure_idx(bilu_mlp* M, size_t count) {
   return BILU_OK;
 }
 
+// Room for the gradient parts of a batch and `steps` losses (at their end).
+bilu_status ensure_work(bilu_mlp* M, int nsample, int steps, int* nrows, float** losses) {
+  int dev = 0, nsm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  *nrows = mlp_train_rows(nsample, nsm);
+  const size_t parts = mlp_train_work(*nrows), need = parts + (size_t)steps * sizeof(float);
+  if (need > M->work_cap) {
+    if (M->work) cudaFree(M->work);
+    M->work = nullptr;
+    M->work_cap = 0;
+    cudaError_t e = cudaMalloc((void**)&M->work, need);
+    if (e != cudaSuccess) return set_error(BILU_ERR_ALLOC, "mlp gradient parts");
+    M->work_cap = need;
+  }
+  *losses = M->work + parts / sizeof(float);
+  return BILU_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -102,7 +122,6 @@ bilu_status bilu_mlp_create(bilu_mlp** out, uint64_t seed) {
   if (e == cudaSuccess) e = cudaMalloc((void**)&M->v, NP * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc((void**)&M->g, NP * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&M->pbf, NP * 2);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&M->loss, sizeof(float));
   if (e == cudaSuccess) e = cudaMemcpy(M->p, h.data(), NP * sizeof(float), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(M->m, 0, NP * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(M->v, 0, NP * sizeof(float));
@@ -124,9 +143,9 @@ bilu_status bilu_mlp_destroy(bilu_mlp* M) {
   cudaFree(M->v);
   cudaFree(M->g);
   cudaFree(M->pbf);
-  cudaFree(M->loss);
   cudaFree(M->stats);
   cudaFree(M->idx);
+  cudaFree(M->work);
   delete M;
   return BILU_OK;
 }
@@ -155,19 +174,16 @@ bilu_status bilu_mlp_train(bilu_mlp* M, const bilu_plan* P, int nsys, const doub
   bilu_status st = check_plan(P);
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
-  float *rown, *coln, *corr;
+  float *rown, *coln, *corr, *d_losses;
+  int nrows;
   st = ensure_stats(M, P, nsys, &rown, &coln, &corr);
+  if (!st) st = ensure_work(M, batch, steps, &nrows, &d_losses);
   if (st) return st;
   cudaError_t e = launch_mlp_rowstats(P->dp, nsys, d_values, rown, coln, corr, s);
-  std::vector<float> losses(steps, 0.0f);
-  float* d_losses = nullptr;
-  if (e == cudaSuccess && steps > 0) e = cudaMalloc((void**)&d_losses, steps * sizeof(float));
-  if (e == cudaSuccess && steps > 0) e = cudaMemsetAsync(d_losses, 0, steps * sizeof(float), s);
   for (int t = 0; t < steps && e == cudaSuccess; ++t) {
-    e = cudaMemsetAsync(M->g, 0, kMlpParams * sizeof(float), s);
-    if (e == cudaSuccess)
-      e = launch_mlp_train(P->dp, nsys, d_values, d_lu_target, rown, coln, corr, M->pbf, batch, nullptr,
-                           seed ^ (0xA24BAED4963EE407ull * (uint64_t)(M->step + 1)), M->g, d_losses + t, s);
+    e = launch_mlp_train(P->dp, nsys, d_values, d_lu_target, rown, coln, corr, M->pbf, batch, nullptr,
+                         seed ^ (0xA24BAED4963EE407ull * (uint64_t)(M->step + 1)), M->work, nrows, M->g, d_losses + t,
+                         s);
     if (e == cudaSuccess) {
       ++M->step;
       // cosine decay from lr to lr / 20 over the call's steps
@@ -178,7 +194,6 @@ bilu_status bilu_mlp_train(bilu_mlp* M, const bilu_plan* P, int nsys, const doub
   if (e == cudaSuccess && steps > 0 && h_losses)
     e = cudaMemcpyAsync(h_losses, d_losses, steps * sizeof(float), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(d_losses);
   return e == cudaSuccess ? BILU_OK : fail(e, "bilu_mlp_train");
 }
 
@@ -190,19 +205,19 @@ bilu_status bilu_mlp_loss_grad(bilu_mlp* M, const bilu_plan* P, int nsys, const 
   bilu_status st = check_plan(P);
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
-  float *rown, *coln, *corr;
+  float *rown, *coln, *corr, *d_loss;
+  int nrows;
   st = ensure_stats(M, P, nsys, &rown, &coln, &corr);
   if (!st) st = ensure_idx(M, nsample);
+  if (!st) st = ensure_work(M, nsample, 1, &nrows, &d_loss);
   if (st) return st;
   cudaError_t e = cudaMemcpyAsync(M->idx, h_idx, nsample * sizeof(int), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = launch_mlp_rowstats(P->dp, nsys, d_values, rown, coln, corr, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(M->g, 0, kMlpParams * sizeof(float), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(M->loss, 0, sizeof(float), s);
   if (e == cudaSuccess)
-    e = launch_mlp_train(P->dp, nsys, d_values, d_lu_target, rown, coln, corr, M->pbf, nsample, M->idx, 0, M->g,
-                         M->loss, s);
+    e = launch_mlp_train(P->dp, nsys, d_values, d_lu_target, rown, coln, corr, M->pbf, nsample, M->idx, 0, M->work,
+                         nrows, M->g, d_loss, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h_grad, M->g, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h_loss, M->loss, sizeof(float), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h_loss, d_loss, sizeof(float), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return e == cudaSuccess ? BILU_OK : fail(e, "bilu_mlp_loss_grad");
 }

@@ -221,6 +221,8 @@ constexpr int TR_X = TR_BWV + H * 8, TR_G1 = TR_X + TB * NF * 4, TR_RED = TR_G1 
 constexpr int TR_SMEM = TR_RED + 3 * 4 * H * 4;
 constexpr uint32_t kTrainTmemCols = 256;  // D1 pre2 | D2 dh1 | D3, D4 the two halves of dW2
 static_assert(TR_W1 % 16 == 0 && TR_X % 16 == 0, "aligned blocks");
+constexpr int kTrainRow = (kMlpParams + 1 + 3) & ~3;  // floats of a block's row: the gradient, the loss
+static_assert(OW2 % 4 == 0 && H * LD * 4 <= TB * TB * 2, "dW2 rows");
 
 // One forward + backward pass over a block of 128 samples (thread = sample) with
 // the three 64-wide GEMMs on the tensor cores (tcgen05.mma, BF16 operands
@@ -232,17 +234,20 @@ static_assert(TR_W1 % 16 == 0 && TR_X % 16 == 0, "aligned blocks");
 // Layer 1, the activations and the output layer run on the CUDA cores in FP32
 // with the accurate tanh.  Per-unit sums over the block (db1, db2, dW3) are
 // reduce-scattered across each warp; dW1 is reduced over the block in shared
-// memory; everything is added to `grad` (FP32 atomics), the summed squared
-// error to `loss`.  Samples: explicit global entry indices (s*nnz+e) or, when
-// idx == NULL, hashed from (seed, sample number).  A tensor-core round that
-// does not complete within the bounded wait adds NaN to `loss` and ends the
-// block.
+// memory; the block's share of the gradient and of the loss is row blockIdx.x
+// of `rows` (kTrainRow floats: the gradient, then the loss), which k_grad_sum
+// adds up in a fixed order.  (Atomic additions to one gradient gave other bits
+// on every run: a parameter on a BF16 rounding boundary then moves the losses
+// of the steps that follow, by 1e-7 to 4e-5 over 40 steps.)  Samples: explicit
+// global entry indices (s*nnz+e) or, when idx == NULL, hashed from (seed,
+// sample number).  A tensor-core round that does not complete within the
+// bounded wait leaves a row of zeros with the loss NaN and ends the block.
 __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, const double* __restrict__ A,
                                                   const double* __restrict__ LUt, const float* __restrict__ rown,
                                                   const float* __restrict__ coln, const float* __restrict__ corr,
                                                   const __nv_bfloat16* __restrict__ pbf, int nsample,
                                                   const int* __restrict__ idx, uint64_t seed, float scale,
-                                                  float* __restrict__ grad, float* __restrict__ loss) {
+                                                  long long first, float* __restrict__ rows) {
   extern __shared__ __align__(1024) unsigned char smt[];
   __shared__ uint64_t s_mbar;
   __shared__ uint32_t s_tmem;
@@ -286,8 +291,9 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
   const float2* bwv = reinterpret_cast<const float2*>(smt + TR_BWV);
   const float b3 = __bfloat162float(pbf[OB3]);
   // ---- sample, features, target
-  const long long q = (long long)blockIdx.x * TB + t;
+  const long long q = first + (long long)blockIdx.x * TB + t;
   const bool live = q < nsample;
+  float* grad = rows + (size_t)blockIdx.x * kTrainRow;
   float f[NF];
   float ytrue = 0.0f;
   if (live) {
@@ -357,9 +363,7 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
   if (!tc::mbar_wait(&s_mbar, 0, kWaitLimit)) s_fail = 1;  // 1 + the parity of the phase that did not complete
   tc::fence_after_sync();
   __syncthreads();
-  if (s_fail) {
-    if (t == 0) atomicAdd(loss, __int_as_float(0x7fc00000));
-  } else {
+  if (!s_fail) {
     // ---- output layer, loss, dout
     float out = b3;
 #pragma unroll 1
@@ -451,9 +455,7 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
     if (!tc::mbar_wait(&s_mbar, 1, kWaitLimit)) s_fail = 2;
     tc::fence_after_sync();
     __syncthreads();
-    if (s_fail) {
-      if (t == 0) atomicAdd(loss, __int_as_float(0x7fc00000));
-    } else {
+    if (!s_fail) {
       // ---- dpre1 = dh1 * gelu'(pre1) into G1; per-unit sums of dpre1 (db1)
       float rs_db1[2];
 #pragma unroll 1
@@ -475,27 +477,40 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
       }
       RED[(2 * 4 + warp) * H + lane] = rs_db1[0];
       RED[(2 * 4 + warp) * H + 32 + lane] = rs_db1[1];
-      // ---- dW2: row r of D3 + D4 is unit r % 64's share (high part for r < 64, low part above)
-      {
-        const int u = (32 * warp + lane) & 63;
+      // ---- dW2: row r of D3 + D4 is unit r % 64's share (high part for r < 64, low part above); the low
+      // parts go through shared memory (AT's, which the tensor cores have read)
+      float* W2L = reinterpret_cast<float*>(smt + TR_AT) + (t & 63) * LD;
+      auto dw2 = [&](auto put) {
 #pragma unroll 1
         for (int c = 0; c < H / 16; ++c) {
           float d3[16], d4[16];
           tc::ld16(trow + 128 + 16 * c, d3);
           tc::ld16(trow + 192 + 16 * c, d4);
-#pragma unroll
-          for (int k = 0; k < 16; ++k) atomicAdd(grad + OW2 + u * H + 16 * c + k, d3[k] + d4[k]);
+          put(16 * c, d3, d4);
         }
-      }
+      };
+      if (warp >= 2)
+        dw2([&](int o, const float(&d3)[16], const float(&d4)[16]) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) W2L[o + k] = d3[k] + d4[k];
+        });
       __syncthreads();
+      if (warp < 2)
+        dw2([&](int o, const float(&d3)[16], const float(&d4)[16]) {
+#pragma unroll
+          for (int k = 0; k < 16; k += 4)
+            *reinterpret_cast<float4*>(grad + OW2 + t * H + o + k) =
+                make_float4((d3[k] + d4[k]) + W2L[o + k], (d3[k + 1] + d4[k + 1]) + W2L[o + k + 1],
+                            (d3[k + 2] + d4[k + 2]) + W2L[o + k + 2], (d3[k + 3] + d4[k + 3]) + W2L[o + k + 3]);
+        });
       if (t == 0) {
         float a = 0.0f, d = 0.0f;
         for (int w = 0; w < TB / 32; ++w) {
           a += s_loss[w];
           d += s_do[w];
         }
-        atomicAdd(loss, a * scale);
-        atomicAdd(grad + OB3, d);
+        grad[kMlpParams] = a * scale;
+        grad[OB3] = d;
       }
       if (t < H) {
         float db2 = 0.0f, dw3 = 0.0f, db1 = 0.0f;
@@ -504,24 +519,69 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
           dw3 += RED[(1 * 4 + w) * H + t];
           db1 += RED[(2 * 4 + w) * H + t];
         }
-        atomicAdd(grad + OB2 + t, db2);
-        atomicAdd(grad + OW3 + t, dw3);
-        atomicAdd(grad + OB1 + t, db1);
+        grad[OB2 + t] = db2;
+        grad[OW3 + t] = dw3;
+        grad[OB1 + t] = db1;
       }
       for (int k = t; k < H * NF; k += TB) {  // dW1[u][f] = sum_t dpre1[t][u] * x[t][f]
         const int u = k / NF, fi = k % NF;
         float acc = 0.0f;
         for (int r = 0; r < TB; ++r) acc = fmaf(G1[r * LD + u], X[r * NF + fi], acc);
-        atomicAdd(grad + OW1 + k, acc);
+        grad[OW1 + k] = acc;
       }
     }
   }
+  if (s_fail)
+    for (int k = t; k < kTrainRow; k += TB) grad[k] = k == kMlpParams ? __int_as_float(0x7fc00000) : 0.0f;
   // a round that timed out may still be in flight: wait once more (bounded) before freeing its columns
   if (s_fail) tc::mbar_wait(&s_mbar, (uint32_t)(s_fail - 1), kWaitLimit);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   if (warp == 0) tc::dealloc(tmem, kTrainTmemCols);
+}
+
+// The gradient and the loss from the blocks' rows, in an order that only the
+// number of rows sets: warp w of a CTA adds rows w, w + 16, ... of 32 columns,
+// one column per lane, then the first warp adds the 16 sums.  Every addition
+// keeps its rounding error (Knuth's two-sum), so the result is the sum's
+// correctly rounded value but for a few ulps of the errors' own sum: nearer to
+// it than any order of plain additions.  acc / cor: the sum and its error so
+// far, continued over the parts of a large batch (start: its first part).
+// Reads 19.5 KB per row: 512 rows (65536 samples) about 4 us.
+constexpr int kSumWarps = 16;
+__device__ __forceinline__ void two_sum(float& s, float& c, float x) {
+  const float t = s + x, z = t - s;
+  c += (s - (t - z)) + (x - z);
+  s = t;
+}
+__global__ void __launch_bounds__(32 * kSumWarps) k_grad_sum(const float* __restrict__ rows, int nrows, int start,
+                                                            float* __restrict__ acc, float* __restrict__ cor,
+                                                            float* __restrict__ grad, float* __restrict__ loss) {
+  __shared__ float s_s[kSumWarps][32], s_c[kSumWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
+  float s = 0.0f, c = 0.0f;
+  if (k <= kMlpParams) {
+#pragma unroll 8
+    for (int r = warp; r < nrows; r += kSumWarps) two_sum(s, c, __ldg(rows + (size_t)r * kTrainRow + k));
+  }
+  s_s[warp][lane] = s;
+  s_c[warp][lane] = c;
+  __syncthreads();
+  if (warp != 0 || k > kMlpParams) return;
+  s = start ? 0.0f : acc[k];
+  c = start ? 0.0f : cor[k];
+  for (int w = 0; w < kSumWarps; ++w) {
+    two_sum(s, c, s_s[w][lane]);
+    c += s_c[w][lane];
+  }
+  acc[k] = s;
+  cor[k] = c;
+  const float v = isfinite(s) ? s + c : s;  // the error of an infinite sum is NaN
+  if (k < kMlpParams)
+    grad[k] = v;
+  else
+    *loss = v;
 }
 
 // Adam on the FP32 master parameters; refreshes the BF16 copy.
@@ -839,16 +899,26 @@ size_t mlp_train_smem() { return TR_SMEM; }
 
 cudaError_t launch_mlp_train(const DevPattern& p, int nsys, const double* A, const double* LUt, const float* rown,
                              const float* coln, const float* corr, const void* pbf, int nsample, const int* idx,
-                             uint64_t seed, float* grad, float* loss, cudaStream_t st) {
+                             uint64_t seed, float* work, int nrows, float* grad, float* loss, cudaStream_t st) {
   if (nsample == 0) return cudaSuccess;
   const size_t smem = mlp_train_smem();
   cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_mlp_train<<<(nsample + TB - 1) / TB, TB, smem, st>>>(p, nsys, A, LUt, rown, coln, corr,
-                                                         (const __nv_bfloat16*)pbf, nsample, idx, seed,
-                                                         1.0f / (float)nsample, grad, loss);
+  float *acc = work, *cor = work + kTrainRow, *rows = work + 2 * kTrainRow;
+  const long long blocks = ((long long)nsample + TB - 1) / TB;
+  for (long long b = 0; b < blocks; b += nrows) {
+    const int part = (int)std::min<long long>(nrows, blocks - b);
+    k_mlp_train<<<part, TB, smem, st>>>(p, nsys, A, LUt, rown, coln, corr, (const __nv_bfloat16*)pbf, nsample, idx,
+                                        seed, 1.0f / (float)nsample, b * TB, rows);
+    k_grad_sum<<<(kMlpParams + 32) / 32, 32 * kSumWarps, 0, st>>>(rows, part, b == 0, acc, cor, grad, loss);
+  }
   return cudaGetLastError();
 }
+
+// Rows of the gradient parts kept at a time: one per block, at most eight per SM (24 MB), whole waves of the
+// training kernel's one CTA per SM.
+int mlp_train_rows(int nsample, int nsm) { return (int)std::min(((long long)nsample + TB - 1) / TB, 8LL * nsm); }
+size_t mlp_train_work(int nrows) { return (size_t)(nrows + 2) * kTrainRow * sizeof(float); }
 
 cudaError_t launch_mlp_adam(float* p, float* m, float* v, const float* g, void* pbf, int count, float lr, int step,
                             cudaStream_t st) {
