@@ -630,10 +630,15 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
       for (int k = tid; k < nnz; k += nt) LUd[k] = __ldg(Ag + k);
       __syncthreads();
       if constexpr (MC > 0) {
+        // without a compact ILU program (dependency pairs off the diagonals: pentadiagonal matrices, the
+        // triangular lattice) the general one, which the plan of a merged form with n <= 1024 always has.
+        // ilu_rows instead: 2048 pentadiagonal systems of 256 rows, FAST order, 1.73 -> 1.83 ms
         if (P.ic_hdr)
           ilu_compact_rows<MC>(P, LUd, sph, a.approach, tid, nt);
-        else
+        else if constexpr (WIDE)
           ilu_rows(P, LUd, a.approach);
+        else
+          ilu_program_rows(P, LUd, a.approach, tid, nt);
       } else {
         if (P.ilu_prog && P.ilu_prog_approach == a.approach)
           ilu_program_rows(P, LUd, a.approach, tid, nt);
