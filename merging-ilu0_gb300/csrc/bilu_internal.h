@@ -367,10 +367,10 @@ cudaError_t launch_expand(const DevPattern& p, int nsys, const double* vin, doub
 cudaError_t launch_ilu0(const DevPattern& p, int nsys, const double* A, double* lu, int approach, int threads,
                         cudaStream_t st);
 cudaError_t launch_parilu0(const DevPattern& p, int nsys, const double* A, const double* init, double* lu,
-                           int sweeps, int threads, cudaStream_t st, double res_tol = 0.0, int* sweeps_out = nullptr,
-                           double* res_out = nullptr, int fast = 0);
+                           int sweeps, int threads, int nsm, cudaStream_t st, double res_tol = 0.0,
+                           int* sweeps_out = nullptr, double* res_out = nullptr, int fast = 0);
 cudaError_t launch_isai(const DevPattern& p, int nsys, const double* lu, void* ail, void* aiu, int fp32,
-                        int threads, cudaStream_t st, int fast = 0);
+                        int threads, int nsm, cudaStream_t st, int fast = 0);
 cudaError_t launch_dense_solve(const DevPattern& p, int nsample, const int* sys_ids, const double* A, const double* b,
                                double* work, double* x_out, cudaStream_t st);
 cudaError_t launch_mlp_rowstats(const DevPattern& p, int nsys, const double* A, float* rown, float* coln, float* corr,

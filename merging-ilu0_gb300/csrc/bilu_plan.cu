@@ -1223,14 +1223,15 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
       if (prec == BILU_PRECOND_ILU0_SPLIT || prec == BILU_PRECOND_ILU0_ISAI)
         e = launch_ilu0(P->dp, nsys, fv, lu, o.ilu_approach, ft, st);
       else
-        e = launch_parilu0(P->dp, nsys, fv, lu_init, lu, o.parilu_sweeps, ft, st, o.parilu_res_tol,
+        e = launch_parilu0(P->dp, nsys, fv, lu_init, lu, o.parilu_sweeps, ft, P->nsm, st, o.parilu_res_tol,
                            R ? R->parilu_sweeps : nullptr, R ? R->ilu_residual : nullptr,
                            o.reduction == BILU_REDUCE_FAST ? 1 : 0);
       if (e != cudaSuccess) return cuda_err(e, "factorisation");
       if (is_isai(prec)) {
         void* ail = ws + sc.ail;
         void* aiu = ws + sc.aiu;
-        e = launch_isai(P->dp, nsys, lu, ail, aiu, fp32 ? 1 : 0, ft, st, o.reduction == BILU_REDUCE_FAST ? 1 : 0);
+        e = launch_isai(P->dp, nsys, lu, ail, aiu, fp32 ? 1 : 0, ft, P->nsm, st,
+                        o.reduction == BILU_REDUCE_FAST ? 1 : 0);
         if (e != cudaSuccess) return cuda_err(e, "isai");
         a.prec = PK_ISAI;
         a.ail = ail;
@@ -1359,7 +1360,7 @@ bilu_status bilu_parilu0(const bilu_plan* Pc, int nsys, const double* d_values, 
     if (e != cudaSuccess) return cuda_err(e, "expand");
     fv = (const double*)P->ws;
   }
-  cudaError_t e = launch_parilu0(P->dp, nsys, fv, d_lu_init, d_lu, sweeps, fact_threads(P), st);
+  cudaError_t e = launch_parilu0(P->dp, nsys, fv, d_lu_init, d_lu, sweeps, fact_threads(P), P->nsm, st);
   return e == cudaSuccess ? BILU_OK : cuda_err(e, "parilu0");
 }
 
@@ -1375,7 +1376,7 @@ bilu_status bilu_isai(const bilu_plan* P, int nsys, const double* d_lu, double* 
   if (!P->has_isai) return set_error(BILU_ERR_INVALID, "bilu_isai: plan was not created with an ISAI preconditioner");
   cudaError_t e = P->general_isai
                       ? launch_isai_general(P->dp, nsys, d_lu, d_ail, 0, fact_threads(P), (cudaStream_t)stream)
-                      : launch_isai(P->dp, nsys, d_lu, d_ail, d_aiu, 0, fact_threads(P), (cudaStream_t)stream,
+                      : launch_isai(P->dp, nsys, d_lu, d_ail, d_aiu, 0, fact_threads(P), P->nsm, (cudaStream_t)stream,
                                     P->opts.reduction == BILU_REDUCE_FAST ? 1 : 0);
   return e == cudaSuccess ? BILU_OK : cuda_err(e, "isai");
 }

@@ -128,10 +128,10 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 
 // fast = true (BILU_REDUCE_FAST): the entries below the diagonal are
 // multiplied by reciprocals of the current diagonal, formed once per sweep,
-// instead of divided; otherwise the quotient by u_jj is formed from the same
-// reciprocal (ifp::quot, the value of the division, in five FP64
-// instructions instead of ten or so).  recips: the n reciprocals fit beside
-// the two iterates (always, but for systems at the shared-memory limit).
+// instead of divided; otherwise, with RECIP, the quotient by u_jj is formed
+// from the same reciprocal (ifp::quot, the value of the division, in five FP64
+// instructions instead of ten or so), else divided: the same value
+// (launch_parilu0 chooses).
 // TRACK: the ILU residual is formed (res_tol > 0 or res_out); a kernel of its
 // own, because FP64 instructions skipped under a runtime condition are
 // if-converted into predicated instructions that still take their FP64-unit
@@ -139,11 +139,11 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // non-tracking sweeps, before this split).
 // SMALL: CTAs of at most 384 threads (n <= 384), bounded for four CTAs per SM
 // instead of two (the per-entry register caches below do not fit it).
-template <bool FAST, bool TRACK, bool SMALL>
+template <bool FAST, bool RECIP, bool TRACK, bool SMALL>
 __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
     k_parilu0(const DevPattern P, int nsys, const double* __restrict__ A, const double* __restrict__ init,
               double* __restrict__ LUout, int sweeps, double res_tol, int* __restrict__ sweeps_out,
-              double* __restrict__ res_out, const int recips) {
+              double* __restrict__ res_out) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[33];
   const int sys = blockIdx.x;
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
   // (instead of three arrays) fit two CTAs per SM at n = 1000
   double* cur = reinterpret_cast<double*>(smem);
   double* nxt = cur + nnz;
-  double* rinv = nxt + nnz;  // n reciprocals of the diagonal (not with !recips)
+  double* rinv = nxt + nnz;  // FAST or RECIP: n reciprocals of the diagonal
   const double* __restrict__ Ag = A + (size_t)sys * nnz;
   const double* Ig = init ? init + (size_t)sys * nnz : Ag;
   double anorm2 = 0.0;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
     double r2 = 0.0;
     const bool last = (it == sweeps);
     if (!TRACK && last) break;
-    if ((FAST || recips) && !last) {
+    if ((FAST || RECIP) && !last) {
       // the correctly rounded reciprocal, the same value as 1.0 / u, by integer arithmetic (ifp::rcp): off
       // the FP64 unit, which the sweeps' FMAs and products keep busy
       auto recip = [](double u) { return FAST ? ifp::rcp(u) : ifp::quot_rcp(u); };
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
     }
     auto ref_quot = [&](double a, int j) {
       const double u = cur[__ldg(P.diag + j)];
-      return recips ? ifp::quot(a, u, rinv[j]) : ifp::quot_slow(a, u);
+      return RECIP ? ifp::quot(a, u, rinv[j]) : a / u;
     };
     // entries with dependency pairs (most pairs first, so a warp's lanes run
     // alike), read from the warp-blocked program: the words of a slot do not
@@ -365,14 +365,13 @@ __global__ void __launch_bounds__(SMALL ? 384 : 512, SMALL ? 4 : 2)
 // as 1.0 / u) instead of divided -- one FP64 reciprocal per row instead of a
 // division per aiU entry.  The unit-diagonal aiL is unchanged.  In the
 // reference order the quotients are formed from the same reciprocals
-// (ifp::quot: five FP64 instructions instead of a division's ten or so) where
-// they fit beside the values (recips; always, but for systems at the
-// shared-memory limit).  ifp::quot_t with the n tails beside them, one FP64
+// (ifp::quot: five FP64 instructions instead of a division's ten or so) with
+// RECIP, else divided: the same values (launch_isai chooses).  ifp::quot_t with the n tails beside them, one FP64
 // instruction less, is slower: they take L1 from the factors (ParILU(5) + ISAI
 // of 1024 3D 10x10x10 systems 451 against 423 us).
-template <typename FT, bool FAST>
+template <typename FT, bool FAST, bool RECIP>
 __global__ void __launch_bounds__(512) k_isai(const DevPattern P, int nsys, const double* __restrict__ LUg,
-                                              FT* __restrict__ ail, FT* __restrict__ aiu, const int recips) {
+                                              FT* __restrict__ ail, FT* __restrict__ aiu) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int sys = blockIdx.x;
   if (sys >= nsys) return;
@@ -405,8 +404,8 @@ __global__ void __launch_bounds__(512) k_isai(const DevPattern P, int nsys, cons
   for (int k = threadIdx.x; k < P.ail_nnz; k += blockDim.x) ail[(size_t)sys * P.ail_nnz + k] = (FT)M[k];
   __syncthreads();
   // ---- aiU
-  double* rinv = M + (P.ail_nnz > P.aiu_nnz ? P.ail_nnz : P.aiu_nnz);  // n reciprocals
-  if (FAST || recips) {
+  double* rinv = M + (P.ail_nnz > P.aiu_nnz ? P.ail_nnz : P.aiu_nnz);  // FAST or RECIP: n reciprocals
+  if (FAST || RECIP) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       const double u = LU[__ldg(P.diag + i)];
       rinv[i] = FAST ? ifp::rcp(u) : ifp::quot_rcp(u);
@@ -417,7 +416,7 @@ __global__ void __launch_bounds__(512) k_isai(const DevPattern P, int nsys, cons
     const int i = __ldg(P.aiu_perm + sl);
     const int beg = __ldg(P.aiu_rp + i), sz = __ldg(P.aiu_rp + i + 1) - beg;
     double* m = M + beg;
-    m[0] = FAST ? rinv[i] : ifp::rcp(LU[__ldg(P.diag + i)]);
+    m[0] = FAST ? rinv[i] : RECIP ? ifp::rcp(LU[__ldg(P.diag + i)]) : 1.0 / LU[__ldg(P.diag + i)];
     int q = __ldg(P.aiu_prog_ptr + (sl >> 5)) + (sl & 31);
     for (int blk = 1; blk < sz; ++blk) {
       const int h = __ldg(P.aiu_prog + q);  // t | count << 5; a row's words are 32 apart
@@ -434,7 +433,7 @@ __global__ void __launch_bounds__(512) k_isai(const DevPattern P, int nsys, cons
         m[ht] = acc * rinv[jt];
       } else {
         const double u = LU[__ldg(P.diag + jt)];
-        m[ht] = recips ? ifp::quot(acc, u, rinv[jt]) : ifp::quot_slow(acc, u);
+        m[ht] = RECIP ? ifp::quot(acc, u, rinv[jt]) : acc / u;
       }
     }
   }
@@ -473,7 +472,7 @@ __device__ __forceinline__ float isai_block_f32(const int* __restrict__ prog, in
 // FP32 arithmetic); the FP64 pipe only rounds the factors.  No reference
 // counterpart (the library's definition; orc_isai_values_ex mode 2).
 __global__ void __launch_bounds__(512) k_isai_f32(const DevPattern P, int nsys, const double* __restrict__ LUg,
-                                                  float* __restrict__ ail, float* __restrict__ aiu, int) {
+                                                  float* __restrict__ ail, float* __restrict__ aiu) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int sys = blockIdx.x;
   if (sys >= nsys) return;
@@ -695,38 +694,60 @@ cudaError_t launch_ilu0(const DevPattern& p, int nsys, const double* A, double* 
   return cudaGetLastError();
 }
 
+// Whether a batch in the reference's order forms its quotients from reciprocals (the same values either way): where
+// the FP64 pipe is the bound, that is with more systems than SMs and at least 256 rows per SM.  Below that a system
+// waits for latencies, which the reciprocals (a chain of integer steps, and a barrier per sweep) add to, unless its
+// threads have several rows each, whose divisions are a longer chain (`alone`).  Nor where the reciprocals would cost
+// a resident CTA (smem: bytes without them; cap: CTAs per SM that the registers admit).  Microseconds, divided / from
+// reciprocals, ParILU(5): 1 system of 6x6 10.6 / 12.4, 16x16 17.6 / 17.8, 31x31 35.7 / 33.0; 6x6, 1024 systems 13.1 /
+// 14.0, 4096 33.3 / 28.4; 10x10, 304 systems 15.0 / 15.8, 608 18.6 / 18.0; 31x31, 304 systems 58.5 / 48.6.  ISAI
+// 23x25, 152 systems 16.4 / 16.6, 608 28.5 / 25.6.  ParILU(2) of 304 systems of 7000 entries, whose reciprocals leave
+// one CTA per SM instead of two, 46.1 / 51.6.
+static bool quotients_from_recips(int n, int nsys, int nsm, long long smem, int cap, bool alone) {
+  if (!fits_smem(smem + 8LL * n)) return false;
+  if (nsys <= nsm) return alone;
+  auto ctas = [&](long long bytes) { return std::min<long long>(cap, (solve_max_smem() + 1024) / (bytes + 1024 + 512)); };
+  return (long long)nsys * n >= 256LL * nsm && ctas(smem + 8LL * n) == ctas(smem);
+}
+
+template <bool FAST, bool RECIP>
+static auto parilu0_kernel(bool track, bool small) {
+  return small ? (track ? k_parilu0<FAST, RECIP, true, true> : k_parilu0<FAST, RECIP, false, true>)
+               : (track ? k_parilu0<FAST, RECIP, true, false> : k_parilu0<FAST, RECIP, false, false>);
+}
+
 cudaError_t launch_parilu0(const DevPattern& p, int nsys, const double* A, const double* init, double* lu,
-                           int sweeps, int threads, cudaStream_t st, double res_tol, int* sweeps_out,
+                           int sweeps, int threads, int nsm, cudaStream_t st, double res_tol, int* sweeps_out,
                            double* res_out, int fast) {
   if (nsys == 0) return cudaSuccess;
-  const int recips = fast || fits_smem((long long)p.nnz * 16 + p.n * 8LL);
+  const int cap = 65536 / ((threads <= 384 ? 40 : 64) * threads);
+  const bool recips = fast || quotients_from_recips(p.n, nsys, nsm, 16LL * p.nnz, cap, p.n > threads);
   const int smem = p.nnz * 8 * 2 + (recips ? p.n * 8 : 0);
-  const bool track = res_tol > 0.0 || res_out != nullptr;
-  const bool small = threads <= 384;
-  auto k = small ? (fast ? (track ? k_parilu0<true, true, true> : k_parilu0<true, false, true>)
-                         : (track ? k_parilu0<false, true, true> : k_parilu0<false, false, true>))
-                 : (fast ? (track ? k_parilu0<true, true, false> : k_parilu0<true, false, false>)
-                         : (track ? k_parilu0<false, true, false> : k_parilu0<false, false, false>));
+  const bool track = res_tol > 0.0 || res_out != nullptr, small = threads <= 384;
+  auto k = fast     ? parilu0_kernel<true, true>(track, small)
+           : recips ? parilu0_kernel<false, true>(track, small)
+                    : parilu0_kernel<false, false>(track, small);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  k<<<nsys, threads, smem, st>>>(p, nsys, A, init, lu, sweeps, res_tol, sweeps_out, res_out, recips);
+  k<<<nsys, threads, smem, st>>>(p, nsys, A, init, lu, sweeps, res_tol, sweeps_out, res_out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_isai(const DevPattern& p, int nsys, const double* lu, void* ail, void* aiu, int fp32, int threads,
-                        cudaStream_t st, int fast) {
+                        int nsm, cudaStream_t st, int fast) {
   if (nsys == 0) return cudaSuccess;
   const bool f32 = fp32 && fast && !p.l_diag;  // FAST FP32 ISAI: computed in FP32 (k_isai_f32)
   // k_isai_f32 stages the factors rounded to float; k_isai reads the FP64 factors through L1
   const int m = p.ail_nnz > p.aiu_nnz ? p.ail_nnz : p.aiu_nnz;
-  int recips = fast || fits_smem(8LL * (m + p.n));
+  const bool recips = fast || quotients_from_recips(p.n, nsys, nsm, 8LL * m, 2048 / threads, false);
   const int smem = ((f32 ? p.nnz : 0) + m + (recips ? p.n : 0)) * (f32 ? 4 : 8);
-  void* k = f32 ? (void*)k_isai_f32
-                : fp32 ? (fast ? (void*)k_isai<float, true> : (void*)k_isai<float, false>)
-                       : (fast ? (void*)k_isai<double, true> : (void*)k_isai<double, false>);
+  void* k = f32      ? (void*)k_isai_f32
+            : fast   ? (fp32 ? (void*)k_isai<float, true, true> : (void*)k_isai<double, true, true>)
+            : recips ? (fp32 ? (void*)k_isai<float, false, true> : (void*)k_isai<double, false, true>)
+                     : (fp32 ? (void*)k_isai<float, false, false> : (void*)k_isai<double, false, false>);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  void* args[] = {const_cast<DevPattern*>(&p), &nsys, &lu, &ail, &aiu, &recips};
+  void* args[] = {const_cast<DevPattern*>(&p), &nsys, &lu, &ail, &aiu};
   return cudaLaunchKernel(k, dim3(nsys), dim3(threads), args, (size_t)smem, st);
 }
 
