@@ -365,7 +365,7 @@ cudaError_t launch_solve_isai_ref(const SolveArgs& a, int fp32, int maxa, int ma
 size_t solve_max_smem();
 cudaError_t launch_expand(const DevPattern& p, int nsys, const double* vin, double* vout, cudaStream_t st);
 cudaError_t launch_ilu0(const DevPattern& p, int nsys, const double* A, double* lu, int approach, int threads,
-                        cudaStream_t st);
+                        int nsm, cudaStream_t st);
 cudaError_t launch_parilu0(const DevPattern& p, int nsys, const double* A, const double* init, double* lu,
                            int sweeps, int threads, int nsm, cudaStream_t st, double res_tol = 0.0,
                            int* sweeps_out = nullptr, double* res_out = nullptr, int fast = 0);

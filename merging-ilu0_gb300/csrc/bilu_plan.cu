@@ -1221,7 +1221,7 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
     } else {
       double* lu = (double*)(ws + sc.lu);
       if (prec == BILU_PRECOND_ILU0_SPLIT || prec == BILU_PRECOND_ILU0_ISAI)
-        e = launch_ilu0(P->dp, nsys, fv, lu, o.ilu_approach, ft, st);
+        e = launch_ilu0(P->dp, nsys, fv, lu, o.ilu_approach, ft, P->nsm, st);
       else
         e = launch_parilu0(P->dp, nsys, fv, lu_init, lu, o.parilu_sweeps, ft, P->nsm, st, o.parilu_res_tol,
                            R ? R->parilu_sweeps : nullptr, R ? R->ilu_residual : nullptr,
@@ -1341,7 +1341,7 @@ bilu_status bilu_ilu0(const bilu_plan* Pc, int nsys, const double* d_values, dou
     if (e != cudaSuccess) return cuda_err(e, "expand");
     fv = d_lu;
   }
-  e = launch_ilu0(P->dp, nsys, fv, d_lu, approach, fact_threads(P), st);
+  e = launch_ilu0(P->dp, nsys, fv, d_lu, approach, fact_threads(P), P->nsm, st);
   return e == cudaSuccess ? BILU_OK : cuda_err(e, "ilu0");
 }
 

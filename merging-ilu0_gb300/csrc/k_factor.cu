@@ -678,16 +678,24 @@ static cudaError_t launch_ilu0_compact(const DevPattern& p, int nsys, const doub
 }
 
 cudaError_t launch_ilu0(const DevPattern& p, int nsys, const double* A, double* lu, int approach, int threads,
-                        cudaStream_t st) {
+                        int nsm, cudaStream_t st) {
   if (nsys == 0) return cudaSuccess;
   const int smem = p.nnz * 8;
   if (p.ic_hdr && fits_smem((long long)smem + p.n * 8LL))
     return p.tc_mc == 2 ? launch_ilu0_compact<2>(p, nsys, A, lu, approach, smem + p.n * 8, st)
                         : launch_ilu0_compact<3>(p, nsys, A, lu, approach, smem + p.n * 8, st);
-  // as many warps as the widest level has rows: each level ends with a CTA
-  // barrier, and more warps only wait there (23x25: levels of 23 rows on 16
-  // warps, 123 barrier stalls per issue; 16384 systems 3.5 -> 2.2 ms)
-  threads = std::min(threads, (std::max(p.maxw_lo, 1) + 31) / 32 * 32);
+  // Fewer threads where they make room for enough CTAs per SM (32 registers: 2048 threads) that the batch takes fewer
+  // waves; at least as many as the widest level has rows, more as far as that room allows, because they copy the
+  // factors in and out.  Milliseconds, 512 threads / as many as the widest level has rows / this: 2048 systems of a
+  // 20x20 9-point grid 1.19 / 0.81 / 0.75; of a 31x31 triangular lattice, of which shared memory admits four CTAs
+  // whatever their threads, 1.10 / 1.43 / 1.10, 1 system 0.264 / 0.299 / 0.264; 64 scattered systems of 1000 rows
+  // 0.027 / 0.035 / 0.027.
+  const int by_smem = std::max(1, (int)((solve_max_smem() + 1024) / (smem + 1024LL)));
+  const int need = (nsys + nsm - 1) / nsm;
+  auto waves = [&](int t) { return (need + std::min(by_smem, 2048 / t) - 1) / std::min(by_smem, 2048 / t); };
+  const int room = 2048 / std::min(by_smem, need) / 32 * 32;
+  const int narrow = std::min(threads, std::max(32, std::max(room, (p.maxw_lo + 31) / 32 * 32)));
+  if (waves(narrow) < waves(threads)) threads = narrow;
   cudaError_t e = cudaFuncSetAttribute(k_ilu0, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   k_ilu0<<<nsys, threads, smem, st>>>(p, nsys, A, lu, approach);
