@@ -287,10 +287,10 @@ __host__ __device__ inline int rr_red_bytes(int nt) { return (2 * nt + 16) * 8; 
 // same on host and device: pv 0 none, 1 two-triangle ISAI, 2 general ISAI, 3
 // ILU factors (inkernel: the FP64 factorisation slot of the merged form).  The
 // reduction slot comes first, so the rest of the layout does not depend on nt.
-// ref: the reference order, whose FP64 upper solve keeps three values per
-// diagonal (tri_solve; one for n > 1024).
+// ref: 1, the reference order, whose FP64 upper solve keeps three values per
+// diagonal (tri_solve); 2, its form with one, the only one for n > 1024.
 __host__ __device__ inline RRLayout rr_layout_base(int n, int nnz, int pv, bool fp32, bool inkernel, int nt,
-                                                   bool ref = false) {
+                                                   int ref = 0) {
   RRLayout L;
   int off = 0;
   const int fts = fp32 ? 4 : 8;
@@ -304,7 +304,7 @@ __host__ __device__ inline RRLayout rr_layout_base(int n, int nnz, int pv, bool 
   if (pv == 1) take(L.mid, (long long)n * fts);
   if (pv == 3) {
     take(L.F, (long long)nnz * (inkernel ? 8 : fts));
-    take(L.rinv, (long long)n * fts * (ref && !fp32 && n <= 1024 ? 3 : 1));
+    take(L.rinv, (long long)n * fts * (ref == 1 && !fp32 && n <= 1024 ? 3 : 1));
   }
   L.total = off;
   return L;
@@ -344,7 +344,7 @@ cudaError_t launch_uneven(const UnevenArgs& u, int threads, int grid, int fp32, 
                           cudaStream_t st);
 cudaError_t launch_solve(const SolveArgs& a, int threads, int fp32, int reduce_fast, int maxl, cudaStream_t st);
 // register-resident solver: pv 0 none, 1 ISAI of L and U, 2 general ISAI, 3 ILU factors; ref: the reference's
-// operation order; nt: the order's threads per system; occ: the occupancy variant (k_bicgstab_rr_occ, 2 to 4 rows
+// operation order (1, or 2: rr_layout_base); nt: the order's threads per system; occ: the occupancy variant (k_bicgstab_rr_occ, 2 to 4 rows
 // per thread, FAST order); mc: DevPattern::tc_mc
 int rr_rows_per_thread(int n, int nt);  // smallest R in {1, 2, 4, 8} with R * nt >= n, else 0
 int rr_slots(int n, int nt);            // the row slots of the kernels: 3 and 6 too
@@ -458,7 +458,8 @@ struct bilu_plan {
   bool rr_sell = false;  // SpMVs read SELL-32 copies of A (and of aiU) made before the solver launch
   bool rr_occ = false;   // the occupancy variant was asked for (staging bit 4)
   int nsm = 0;           // SMs of the device
-  bilu::RRLayout rr_lay;
+  bilu::RRLayout rr_lay, rr_lean;  // rr_lean: the reference order's layout with one value per diagonal
+  int rr_ctas = 0, rr_lean_ctas = 0;  // resident CTAs per SM with them; 0: none
   // workspace
   void* ws = nullptr;
   size_t ws_bytes = 0;

@@ -490,40 +490,61 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
   // the merged form factorises in FP64 in the factor slot before rounding to FT
   // more systems than are resident at once; fewer may run on more threads (rr_split) with the same layout
   const int split = rr_split(pv, ref ? 1 : 0, n, nt, 1 << 30, P.nsm);
-  RRLayout L = rr_layout_base(n, P.nnz, pv, fp32, pk == PK_ILU_INKERNEL, nt, ref);
-  int off = L.total;
-  auto take = [&](int& dst, long long bytes) {
-    dst = off;
-    off = (int)((off + bytes + 15) & ~15LL);
-  };
-  int dev = 0, per_sm = 0, reserved = 0, optin = 0, occ = 0;
+  int dev = 0, per_sm = 0, reserved = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
   cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const void* k = rr_kernel(pv, fp32 ? 1 : 0, n, nt, ref ? 1 : 0, occ_variant && split == 1 ? 1 : 0, P.tc_mc, split);
-  if (!k) return false;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(optin, off)) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, nt * split, off) != cudaSuccess || occ < 1) {
-    cudaGetLastError();
-    return false;
-  }
-  const int budget = std::min(optin, per_sm / occ - reserved);
-  if (off > budget) return false;
-  auto stage = [&](int& dst, long long bytes, int bit) {
-    if ((mask & bit) && bytes > 0 && off + bytes <= budget) take(dst, bytes);
+  // the layout L for an order (0 FAST, 1 reference, 2 reference with one value per diagonal); returns the resident
+  // CTAs per SM, 0: no such kernel, or it does not fit
+  auto layout = [&](int order, RRLayout& L) {
+    L = rr_layout_base(n, P.nnz, pv, fp32, pk == PK_ILU_INKERNEL, nt, order);
+    int off = L.total, occ = 0;
+    const void* k = rr_kernel(pv, fp32 ? 1 : 0, n, nt, order, occ_variant && split == 1 ? 1 : 0, P.tc_mc, split);
+    if (!k) return 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(optin, off)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, nt * split, off) != cudaSuccess || occ < 1) {
+      cudaGetLastError();
+      return 0;
+    }
+    const int budget = std::min(optin, per_sm / occ - reserved);
+    if (off > budget) return 0;
+    auto stage = [&](int& dst, long long bytes, int bit) {
+      if (!(mask & bit) || bytes <= 0 || off + bytes > budget) return;
+      dst = off;
+      off = (int)((off + bytes + 15) & ~15LL);
+    };
+    stage(L.A, (long long)P.nnz_in * 8, 1);
+    if (pv == 1 || pv == 2) stage(L.ail, (long long)P.ail_rp[n] * fts, 2);
+    if (pv == 1) stage(L.aiu, (long long)P.aiu_rp[n] * fts, 4);
+    L.total = off;
+    return occ;
   };
-  stage(L.A, (long long)P.nnz_in * 8, 1);
-  if (pv == 1 || pv == 2) stage(L.ail, (long long)P.ail_rp[n] * fts, 2);
-  if (pv == 1) stage(L.aiu, (long long)P.aiu_rp[n] * fts, 4);
-  L.total = off;
+  RRLayout L, lean;
+  const int ctas = layout(ref ? 1 : 0, L);
+  // (at up to 4 rows per thread the registers admit fewer CTAs than shared memory)
+  const int lean_ctas = ref && pv == 3 && !fp32 && !wide && rr_slots(n, nt) >= 6 ? layout(2, lean) : 0;
+  if (ctas < 1 && lean_ctas < 1) return false;
   P.rr = true;
   P.rr_threads = nt;
   P.rr_pv = pv;
-  P.rr_lay = L;
+  P.rr_lay = ctas < 1 ? lean : L;
+  P.rr_lean = lean;
+  P.rr_ctas = ctas;
+  P.rr_lean_ctas = lean_ctas;
   P.rr_sell = (mask & 8) != 0 && !P.sa_off.empty();
   P.rr_occ = occ_variant;
   return true;
+}
+
+// Whether a batch in the reference's order runs on the kernel with one value per diagonal (kRefLean): where the
+// smaller layout saves a wave of CTAs (a wave is a few percent slower).  Merged ILU(0), 28x28 9-point grid, three
+// values / one: 256 systems 1.33 / 1.35 ms, 2048 systems 9.30 / 6.97 ms; 1800 pentadiagonal systems of 256 rows
+// 1.56 / 1.10 ms; 2048 2D 16x16 systems, 11 CTAs per SM / 12, 1.70 / 1.81 ms.
+bool rr_takes_lean(const bilu_plan& P, int nsys) {
+  if (P.rr_lean_ctas < 1 || P.rr_ctas < 1) return P.rr_lean_ctas > 0;
+  auto waves = [&](long long per) { return (nsys + per * P.nsm - 1) / (per * P.nsm); };
+  return waves(P.rr_lean_ctas) < waves(P.rr_ctas);
 }
 
 // Default: the caller's threads per system, else the fewest warps that give
@@ -1028,7 +1049,8 @@ bilu_status bilu_plan_autotune(bilu_plan* P, int nsys, const double* d_values, c
   if (st) return st;
   const int base = round_up((P->n + 7) / 8, 32);
   const int keep_nt = P->rr_threads;
-  const RRLayout keep_lay = P->rr_lay;
+  const RRLayout keep_lay = P->rr_lay, keep_lean = P->rr_lean;
+  const int keep_ctas = P->rr_ctas, keep_lean_ctas = P->rr_lean_ctas;
   const bool keep_sell = P->rr_sell, keep_occ = P->rr_occ;
   float best = -1.0f;
   int best_nt = keep_nt, best_mask = -1;
@@ -1061,6 +1083,9 @@ bilu_status bilu_plan_autotune(bilu_plan* P, int nsys, const double* d_values, c
   } else {
     P->rr_threads = keep_nt;
     P->rr_lay = keep_lay;
+    P->rr_lean = keep_lean;
+    P->rr_ctas = keep_ctas;
+    P->rr_lean_ctas = keep_lean_ctas;
     P->rr_sell = keep_sell;
     P->rr_occ = keep_occ;
   }
@@ -1271,10 +1296,11 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
   // the reference's ISAI solvers: several systems per CTA, unless the caller asked for a CTA size
   const bool isai_ref = !P->rr && a.prec == PK_ISAI && !P->general_isai && o.reduction != BILU_REDUCE_FAST &&
                         o.threads_per_system == 0 && isai_ref_fits(P->n, fp32 ? 1 : 0, P->a_maxl, maxi);
+  const bool lean = P->rr && rr_takes_lean(*P, nsys);
   e = isai_ref
           ? launch_solve_isai_ref(a, fp32 ? 1 : 0, P->a_maxl, maxi, P->nsm, st)
-      : P->rr ? launch_solve_rr(a, P->rr_lay, P->rr_threads, P->rr_pv, fp32 ? 1 : 0,
-                              o.reduction == BILU_REDUCE_FAST ? 0 : 1, P->rr_occ ? 1 : 0, P->nsm, st)
+      : P->rr ? launch_solve_rr(a, lean ? P->rr_lean : P->rr_lay, P->rr_threads, P->rr_pv, fp32 ? 1 : 0,
+                              o.reduction == BILU_REDUCE_FAST ? 0 : lean ? 2 : 1, P->rr_occ ? 1 : 0, P->nsm, st)
             : launch_solve(a, P->threads, fp32 ? 1 : 0, o.reduction == BILU_REDUCE_FAST ? 1 : 0, maxl, st);
   if (e != cudaSuccess) return cuda_err(e, "solver launch");
   if (P->timing) cudaEventRecord(P->ev[2], st);

@@ -12,26 +12,26 @@ namespace {
 // l + 32 (w R + k), a block of the reference's lane-strided inner-product
 // terms; the inner products chain through the warps in order (ref_chain_sum),
 // so every scalar is the reference's bit for bit.
-template <int R, int PV, typename FT, bool REF = false>
+template <int R, int PV, typename FT, int ORD>
 __global__ void BILU_RR_BOUNDS k_bicgstab_rr(const SolveArgs a, const RRLayout L) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int sys = blockIdx.x;
   if (sys >= a.nsys) return;
   const DevPattern& P = a.pat;
-  rr_solve<R, PV, FT, true, REF ? kRef : kFast>(a, P, L, smem, sys, a.A + (size_t)sys * P.a_nnz, a.b + (size_t)sys * P.n,
+  rr_solve<R, PV, FT, true, ORD>(a, P, L, smem, sys, a.A + (size_t)sys * P.a_nnz, a.b + (size_t)sys * P.n,
                                  a.x + (size_t)sys * P.n);
 }
 
-template <int PV, typename FT, bool REF>
+template <int PV, typename FT, int ORD>
 const void* rr_kernel_pv(int slots) {
   switch (slots) {
-    case 1: return (const void*)k_bicgstab_rr<1, PV, FT, REF>;
-    case 2: return (const void*)k_bicgstab_rr<2, PV, FT, REF>;
-    case 3: return (const void*)k_bicgstab_rr<3, PV, FT, REF>;
-    case 4: return (const void*)k_bicgstab_rr<4, PV, FT, REF>;
+    case 1: return (const void*)k_bicgstab_rr<1, PV, FT, ORD>;
+    case 2: return (const void*)k_bicgstab_rr<2, PV, FT, ORD>;
+    case 3: return (const void*)k_bicgstab_rr<3, PV, FT, ORD>;
+    case 4: return (const void*)k_bicgstab_rr<4, PV, FT, ORD>;
   }
-  if constexpr (PV == 3 || REF)  // else split (rr_split)
-    return slots == 6 ? (const void*)k_bicgstab_rr<6, PV, FT, REF> : (const void*)k_bicgstab_rr<8, PV, FT, REF>;
+  if constexpr (PV == 3 || ORD != kFast)  // else split (rr_split)
+    return slots == 6 ? (const void*)k_bicgstab_rr<6, PV, FT, ORD> : (const void*)k_bicgstab_rr<8, PV, FT, ORD>;
   return nullptr;
 }
 
@@ -76,14 +76,17 @@ const void* rr_kernel(int pv, int fp32, int n, int nt, int ref, int occ, int mc,
   if (occ) return ref ? nullptr : rr_occ_kernel(pv, fp32, slots);  // FAST order, 2 to 4 rows
   if (pv == 3 && mc) return rr_lu_kernel(fp32, slots, ref, mc);
   if (ref) {  // reference order: no preconditioner or ILU factors
-    if (pv == 0) return rr_kernel_pv<0, double, true>(slots);
-    if (pv == 3) return fp32 ? rr_kernel_pv<3, float, true>(slots) : rr_kernel_pv<3, double, true>(slots);
-    return nullptr;
+    if (pv == 0) return rr_kernel_pv<0, double, kRef>(slots);
+    if (pv != 3) return nullptr;
+    if (ref == kRefLean)  // 5 to 8 rows per thread (rr_configure)
+      return slots == 6 ? (const void*)k_bicgstab_rr<6, 3, double, kRefLean>
+                        : (const void*)k_bicgstab_rr<8, 3, double, kRefLean>;
+    return fp32 ? rr_kernel_pv<3, float, kRef>(slots) : rr_kernel_pv<3, double, kRef>(slots);
   }
-  if (pv == 0) return rr_kernel_pv<0, double, false>(slots);
-  if (pv == 1) return fp32 ? rr_kernel_pv<1, float, false>(slots) : rr_kernel_pv<1, double, false>(slots);
-  if (pv == 3) return fp32 ? rr_kernel_pv<3, float, false>(slots) : rr_kernel_pv<3, double, false>(slots);
-  return fp32 ? rr_kernel_pv<2, float, false>(slots) : rr_kernel_pv<2, double, false>(slots);
+  if (pv == 0) return rr_kernel_pv<0, double, kFast>(slots);
+  if (pv == 1) return fp32 ? rr_kernel_pv<1, float, kFast>(slots) : rr_kernel_pv<1, double, kFast>(slots);
+  if (pv == 3) return fp32 ? rr_kernel_pv<3, float, kFast>(slots) : rr_kernel_pv<3, double, kFast>(slots);
+  return fp32 ? rr_kernel_pv<2, float, kFast>(slots) : rr_kernel_pv<2, double, kFast>(slots);
 }
 
 cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int pv, int fp32, int ref, int occ,

@@ -283,11 +283,14 @@ __device__ __forceinline__ void rows_acc_sell(const VT* __restrict__ val, const 
 // The orders a solver instantiation follows.
 //   kFast    the FAST order (top of this file)
 //   kRef     the reference's operation order
+//   kRefLean the same, with one value per diagonal for the upper solve instead
+//            of three (tri_solve): where that saves a wave of CTAs
+//            (rr_takes_lean), and past 1024 rows
 //   kFastChain  the FAST order of systems past the FAST kernels' 1024 rows,
 //            the shared-memory solver's (k_solve.cu with REF = false): rows and
 //            reciprocals as in FAST, triangular-solve sums, inner products and
 //            the true residual's rows as in the reference
-enum RROrder : int { kFast = 0, kRef = 1, kFastChain = 2 };
+enum RROrder : int { kFast = 0, kRef = 1, kRefLean = 2, kFastChain = 3 };
 
 // Barrier at the end of a level.  WIDE: of the solve's `team` threads, one
 // warp per 32 rows of the widest level (a warp barrier for one warp); the other
@@ -318,13 +321,13 @@ __device__ __forceinline__ void team_sync(int team) {
 // z_i into zd for FP32 factors.  Ends with the team's barrier.
 // ORD != kFast: the reference's order instead (PrecondBiCGSTAB_exact_ilu0_app1_merged_gpu.cu:22-108):
 // s = sum of fma(F, y, s) from 0 in program order, then y_i - s, and for UPPER
-// (y_i - s) / u_ii (kRef with FP64 factors) or (y_i - s) * rinv_i (FP32
-// factors and kFastChain, the library's definitions).  The quotient is formed
-// from the reciprocal (the value of the division, k_intfp.cuh): rinv holds n
-// reciprocals, their n tails and the n u_ii (four FP64 instructions).  WIDE
-// keeps the reciprocals alone (five FP64 instructions, 20 KB less): u_ii is
-// the factor just before the row's upper entries, and where the row has none
-// the program's first entry holds its position.
+// (y_i - s) / u_ii (kRef and kRefLean with FP64 factors) or (y_i - s) * rinv_i
+// (FP32 factors and kFastChain, the library's definitions).  The quotient is
+// formed from the reciprocal (the value of the division, k_intfp.cuh): rinv
+// holds n reciprocals, their n tails and the n u_ii (four FP64 instructions).
+// kRefLean keeps the reciprocals alone (five FP64 instructions, 16 n bytes
+// less): u_ii is the factor just before the row's upper entries, and where the
+// row has none the program's first entry holds its position.
 template <bool UPPER, typename FT, int ORD, bool WIDE>
 __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const int* __restrict__ prog, int nlev,
                                           const FT* __restrict__ F, const FT* __restrict__ rinv, FT* y, double* zd,
@@ -363,12 +366,12 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
       const FT d = y[i] - acc;
       if (UPPER) {
         FT z;
-        if constexpr (sizeof(FT) == 8 && ORD == kRef) {
-          z = WIDE ? ifp::quot(d, F[(e[0] >> SH) - cnt], rinv[i])
-                   : ifp::quot_t(d, rinv[2 * n + i], rinv[i], rinv[n + i]);
-        } else {
+        if constexpr (sizeof(FT) == 8 && ORD == kRef)
+          z = ifp::quot_t(d, rinv[2 * n + i], rinv[i], rinv[n + i]);
+        else if constexpr (sizeof(FT) == 8 && ORD == kRefLean)
+          z = ifp::quot(d, F[(e[0] >> SH) - cnt], rinv[i]);
+        else
           z = d * rinv[i];
-        }
         y[i] = z;
         if (sizeof(FT) == 4) zd[i] = (double)z;
       } else {
@@ -463,7 +466,9 @@ __device__ __forceinline__ void tri_solve_compact(const uint2* __restrict__ prog
     if (ORD != kFast) acc = y[i] - acc;
     if (UPPER) {
       if constexpr (sizeof(FT) == 8 && ORD == kRef)
-        acc = WIDE ? ifp::quot(acc, F[k0 - cnt], rinv[i]) : ifp::quot_t(acc, rinv[2 * n + i], rinv[i], rinv[n + i]);
+        acc = ifp::quot_t(acc, rinv[2 * n + i], rinv[i], rinv[n + i]);
+      else if constexpr (sizeof(FT) == 8 && ORD == kRefLean)
+        acc = ifp::quot(acc, F[k0 - cnt], rinv[i]);
       else
         acc = acc * rinv[i];
       if (sizeof(FT) == 4) zd[i] = (double)acc;
@@ -563,6 +568,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
                                          unsigned char* smem, const int sys, const double* Ag, const double* bg,
                                          double* xg) {
   constexpr bool REF = ORD != kFast;  // inner products in the reference's order, row blocks to match
+  constexpr bool REF_ROWS = ORD == kRef || ORD == kRefLean;
   const int n = P.n, nt = blockDim.x, tid = threadIdx.x, nw = nt >> 5;
   // this thread's rows: rb + k * rs, k < R.  FAST: tid + k * nt, split: the h-th
   // part of order thread t's (split_chain_sum).  REF: lane + 32 (warp R + k), so
@@ -672,10 +678,10 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     __syncthreads();
     for (int i = tid; i < n; i += nt) {
       const double dgi = (double)Fs[__ldg(P.diag + i)];
-      if (ORD == kRef && sizeof(FT) == 8) {  // the upper solve's quotients by u_ii (tri_solve)
+      if (REF_ROWS && sizeof(FT) == 8) {  // the upper solve's quotients by u_ii (tri_solve)
         const double y = ifp::quot_rcp(dgi);
         rinv[i] = (FT)y;
-        if (!WIDE) {
+        if (ORD == kRef) {
           rinv[n + i] = (FT)ifp::quot_tail(dgi, y);
           rinv[2 * n + i] = (FT)dgi;
         }
@@ -796,7 +802,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     __syncthreads();
     BILU_RR_APPLY();  // p_hat in sph
     // v = A p_hat, (r_hat, v)
-    if (ORD == kRef)
+    if (REF_ROWS)
       rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, v, P.a_maxl);
     else if (Asell)
       rows_acc_sell<R>(Asell, saci, P.sa_off, arp, rb, rs, n, sph, v);
@@ -838,7 +844,7 @@ __device__ __forceinline__ void rr_solve(const SolveArgs& a, const DevPattern& P
     }
     BILU_RR_APPLY();  // s_hat in sph
     // t = A s_hat, (t, s), (t, t)
-    if (ORD == kRef)
+    if (REF_ROWS)
       rows_acc_ref<R>(Am, aci, arp, rb, rs, n, sph, t, P.a_maxl);
     else if (Asell)
       rows_acc_sell<R>(Asell, saci, P.sa_off, arp, rb, rs, n, sph, t);

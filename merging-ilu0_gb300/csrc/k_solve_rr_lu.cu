@@ -37,6 +37,9 @@ const void* lu_r(int slots) {
 
 template <int MC>
 const void* lu_mc(int fp32, int slots, int ref) {
+  if (ref == kRefLean)  // 5 to 8 rows per thread (rr_configure)
+    return slots == 6 ? (const void*)k_bicgstab_rr_lu<6, double, kRefLean, MC>
+                      : (const void*)k_bicgstab_rr_lu<8, double, kRefLean, MC>;
   if (ref) return fp32 ? lu_r<float, kRef, MC>(slots) : lu_r<double, kRef, MC>(slots);
   return fp32 ? lu_r<float, kFast, MC>(slots) : lu_r<double, kFast, MC>(slots);
 }

@@ -33,9 +33,9 @@ __global__ void __launch_bounds__(NT, 2) k_bicgstab_rr_wide(const SolveArgs a, c
 template <int PV, typename FT, int MC = 0>
 const void* wide_pv(int ref, int nt) {
   if (nt <= 192)
-    return ref ? (const void*)k_bicgstab_rr_wide<192, PV, FT, kRef, MC>
+    return ref ? (const void*)k_bicgstab_rr_wide<192, PV, FT, kRefLean, MC>
                : (const void*)k_bicgstab_rr_wide<192, PV, FT, kFastChain, MC>;
-  return ref ? (const void*)k_bicgstab_rr_wide<256, PV, FT, kRef, MC>
+  return ref ? (const void*)k_bicgstab_rr_wide<256, PV, FT, kRefLean, MC>
              : (const void*)k_bicgstab_rr_wide<256, PV, FT, kFastChain, MC>;
 }
 
