@@ -196,9 +196,14 @@ void build_levels(bilu_plan& P) {
 }
 
 // Compact solve programs (DevPattern::tc_*), where no row of either triangle
-// has more than three entries.  Their levels are all as wide as the widest one,
-// so a schedule whose levels fill less than a quarter of that keeps the general
-// programs (padding would crowd the words out of L1).
+// has more than three entries.  Their levels are all as wide as the widest one;
+// a schedule that needs more than 9/4 slots per row, more than any 2D or 3D grid
+// does (its levels are the cuts of a box by planes: at most 2.13 slots), keeps
+// the general programs, because padding crowds the words out of L1 and gives
+// threads rounds without a row.  FAST order, 2048 systems, compact / general:
+// scattered patterns, 3.0 slots per row, 1000 rows, ParILU 1.02 / 0.91 ms,
+// 2.5 slots, 200 rows 0.275 / 0.255; triangular lattice 31x31, 2.0 slots, 1.96 /
+// 2.26.
 void build_compact_programs(bilu_plan& P) {
   P.tc_lo.clear();
   P.tc_up.clear();
@@ -207,7 +212,7 @@ void build_compact_programs(bilu_plan& P) {
   for (int i = 0; i < P.n; ++i) mc = std::max({mc, P.diag[i] - P.rp[i], P.rp[i + 1] - 1 - P.diag[i]});
   const long long slots_lo = (long long)(P.lev_lo_ptr.size() - 1) * P.maxw_lo;
   const long long slots_up = (long long)(P.lev_up_ptr.size() - 1) * P.maxw_up;
-  if (mc > 3 || P.nnz >= kCompactMaxNnz || std::max(slots_lo, slots_up) > 4LL * P.n) return;
+  if (mc > 3 || P.nnz >= kCompactMaxNnz || 4 * std::max(slots_lo, slots_up) > 9LL * P.n) return;
   auto fill = [&](const std::vector<int>& ptr, const std::vector<int>& rows, int W, bool upper, std::vector<int>& out) {
     out.assign(2 * (ptr.size() - 1) * (size_t)W, 0);
     for (size_t l = 0; l + 1 < ptr.size(); ++l)
