@@ -542,6 +542,19 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
   return true;
 }
 
+// Whether a batch of systems of more than 1024 rows runs on the shared-memory kernel (the same bits) instead of
+// k_bicgstab_rr_wide: no more systems than SMs, so that its one CTA of 1024 threads per SM is no loss, and nothing for
+// the wide kernel's prefetched level words to gain, because there are no triangular solves or their levels are more
+// than two rounds of its 192 to 256 threads wide.  Not where the caller chose threads or staging.  Milliseconds, wide /
+// shared-memory kernel, FAST order: no preconditioner, 36x36, 1 system 0.281 / 0.232, 152 scattered systems of 1100
+// rows 0.251 / 0.214, 153 of them 0.251 / 0.353; merged ILU(0), scattered, levels of 750 rows, 1 system 0.252 / 0.183,
+// 200 systems 0.347 / 0.377; 36x36 grid, levels of 36 rows, 1 system 0.430 / 1.086.
+bool takes_shared(const bilu_plan& P, int nsys) {
+  const bilu_options& o = P.opts;
+  return P.rr && P.n > 1024 && nsys <= P.nsm && o.threads_per_system == 0 && o.smem_staging < 0 &&
+         (P.rr_pv == 0 || std::max(P.maxw_lo, P.maxw_up) > 2 * P.rr_threads) && P.lay.total <= (int)solve_max_smem();
+}
+
 // Whether a batch in the reference's order runs on the kernel with one value per diagonal (kRefLean): where the
 // smaller layout saves a wave of CTAs (a wave is a few percent slower).  Merged ILU(0), 28x28 9-point grid, three
 // values / one: 256 systems 1.33 / 1.35 ms, 2048 systems 9.30 / 6.97 ms; 1800 pentadiagonal systems of 256 rows
@@ -1304,9 +1317,10 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
   const bool lean = P->rr && rr_takes_lean(*P, nsys);
   e = isai_ref
           ? launch_solve_isai_ref(a, fp32 ? 1 : 0, P->a_maxl, maxi, P->nsm, st)
-      : P->rr ? launch_solve_rr(a, lean ? P->rr_lean : P->rr_lay, P->rr_threads, P->rr_pv, fp32 ? 1 : 0,
-                              o.reduction == BILU_REDUCE_FAST ? 0 : lean ? 2 : 1, P->rr_occ ? 1 : 0, P->nsm, st)
-            : launch_solve(a, P->threads, fp32 ? 1 : 0, o.reduction == BILU_REDUCE_FAST ? 1 : 0, maxl, st);
+      : P->rr && !takes_shared(*P, nsys)
+          ? launch_solve_rr(a, lean ? P->rr_lean : P->rr_lay, P->rr_threads, P->rr_pv, fp32 ? 1 : 0,
+                            o.reduction == BILU_REDUCE_FAST ? 0 : lean ? 2 : 1, P->rr_occ ? 1 : 0, P->nsm, st)
+          : launch_solve(a, P->threads, fp32 ? 1 : 0, o.reduction == BILU_REDUCE_FAST ? 1 : 0, maxl, st);
   if (e != cudaSuccess) return cuda_err(e, "solver launch");
   if (P->timing) cudaEventRecord(P->ev[2], st);
   return BILU_OK;
