@@ -30,7 +30,7 @@ const void* rr_kernel_pv(int slots) {
     case 3: return (const void*)k_bicgstab_rr<3, PV, FT, ORD>;
     case 4: return (const void*)k_bicgstab_rr<4, PV, FT, ORD>;
   }
-  if constexpr (PV == 3 || ORD != kFast)  // else split (rr_split)
+  if constexpr (PV == 3 || PV == 0 || ORD != kFast)  // else split (rr_split)
     return slots == 6 ? (const void*)k_bicgstab_rr<6, PV, FT, ORD> : (const void*)k_bicgstab_rr<8, PV, FT, ORD>;
   return nullptr;
 }
@@ -62,18 +62,32 @@ int rr_max_threads(int R, bool wide) {
 // leave waiting, 0.543 / 0.474 / 0.580.  Past that two, but for 7 or 8 rows on
 // one warp (8192 2D 16x16 systems 1.64 ms on two, 1.47 on four; at 96 and 128
 // threads four are 5 to 15 % slower).
+//
+// Without a preconditioner (pv = 0) the inner products, which a split lengthens,
+// are most of an iteration: at 128 threads four only while each system has an SM
+// to itself, and two instead of one only where the 1024 / (2 nt) CTAs that then
+// share an SM, instead of 384 / nt, save a wave that outweighs a wave's 1.1 to
+// 1.3 times longer time; past four waves the two forms are within 5 % of each
+// other either way.  Microseconds on one / two / four, 31x31: 152 systems 168 /
+// 166 / 154, 304 197 / 209 / 199, 456 243 / 263 / 375, 608 451 / 326 / 389, 800 467
+// / 530 / 567, 2048 1127 / 1156 / 1304; 760 tridiagonal rows, 96 threads: 304 193 /
+// 206 / 187, 1000 488 / 550 / 656, 1500 714 / 651 / 847.
 int rr_split(int pv, int ref, int n, int nt, int nsys, int nsm) {
   const int slots = rr_slots(n, nt);
   if (pv == 3 || ref || slots < 6 || nt > 128) return 1;
-  if (nsys <= (long long)nsm * (1024 / (4 * nt))) return 4;
-  return slots == 8 && nt == 32 ? 4 : 2;
+  if (nsys <= (long long)nsm * (pv == 0 && nt == 128 ? 1 : 1024 / (4 * nt))) return 4;
+  if (slots == 8 && nt == 32) return 4;
+  if (pv != 0) return 2;
+  auto waves = [&](long long per) { return (nsys + per * nsm - 1) / (per * nsm); };
+  const long long one = waves(384 / nt), two = waves(1024 / (2 * nt));
+  return one <= 4 && 10 * one >= 13 * two ? 2 : 1;
 }
 
 const void* rr_kernel(int pv, int fp32, int n, int nt, int ref, int occ, int mc, int split) {
   const int slots = rr_slots(n, nt);
   if (nt > 128 && slots > 4) return occ ? nullptr : rr_wide_kernel(pv, fp32, ref, nt, mc);
   if (split > 1) return rr_split_kernel(pv, fp32, split, slots);
-  if (occ) return ref ? nullptr : rr_occ_kernel(pv, fp32, slots);  // FAST order, 2 to 4 rows
+  if (occ && slots <= 4) return ref ? nullptr : rr_occ_kernel(pv, fp32, slots);  // FAST order, 2 to 4 rows
   if (pv == 3 && mc) return rr_lu_kernel(fp32, slots, ref, mc);
   if (ref) {  // reference order: no preconditioner or ILU factors
     if (pv == 0) return rr_kernel_pv<0, double, kRef>(slots);
