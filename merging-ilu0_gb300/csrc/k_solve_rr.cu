@@ -71,15 +71,16 @@ int rr_max_threads(int R, bool wide) {
 // other either way.  Microseconds on one / two / four, 31x31: 152 systems 168 /
 // 166 / 154, 304 197 / 209 / 199, 456 243 / 263 / 375, 608 451 / 326 / 389, 800 467
 // / 530 / 567, 2048 1127 / 1156 / 1304; 760 tridiagonal rows, 96 threads: 304 193 /
-// 206 / 187, 1000 488 / 550 / 656, 1500 714 / 651 / 847.
+// 206 / 187, 1000 488 / 550 / 656, 1500 714 / 651 / 847.  On one warp one while
+// it is a single wave: 16x16, 1500 systems 241 / 244 / 300, 2048 418 / 335 / 364.
 int rr_split(int pv, int ref, int n, int nt, int nsys, int nsm) {
   const int slots = rr_slots(n, nt);
   if (pv == 3 || ref || slots < 6 || nt > 128) return 1;
   if (nsys <= (long long)nsm * (pv == 0 && nt == 128 ? 1 : 1024 / (4 * nt))) return 4;
-  if (slots == 8 && nt == 32) return 4;
-  if (pv != 0) return 2;
   auto waves = [&](long long per) { return (nsys + per * nsm - 1) / (per * nsm); };
   const long long one = waves(384 / nt), two = waves(1024 / (2 * nt));
+  if (slots == 8 && nt == 32) return pv == 0 && one == 1 ? 1 : 4;
+  if (pv != 0) return 2;
   return one <= 4 && 10 * one >= 13 * two ? 2 : 1;
 }
 

@@ -14,7 +14,7 @@ PATTERNS = {"tri_150": band(150, (-1, 1)), "tri_256": band(256, (-1, 1)), "penta
 
 
 @pytest.mark.parametrize("name", list(PATTERNS))
-@pytest.mark.parametrize("nsys", [1, 152, 153, 305, 457, 609, 1000, 2500])
+@pytest.mark.parametrize("nsys", [1, 152, 153, 305, 457, 609, 1000, 1500, 2500])
 @pytest.mark.parametrize("staging", [-1, 16, 25])
 def test_without_preconditioner(cuda, name, nsys, staging):
     rp, ci = PATTERNS[name]
