@@ -232,19 +232,23 @@ void build_compact_programs(bilu_plan& P) {
   P.tc_mc = std::max(mc, 2);
 }
 
-// Triangular-solve programs (DevPattern::tp_*) from the level schedules; only
-// for the register-resident solver's range.
+// Triangular-solve programs (DevPattern::tp_*) from the level schedules, for
+// the register-resident solver with ILU factors; where there are compact
+// programs, only the FAST order's occupancy variant (n <= 1024) reads them.
 void build_trsv_programs(bilu_plan& P) {
   P.tp_lo_hdr.clear();
   P.tp_lo.clear();
   P.tp_up_hdr.clear();
   P.tp_up.clear();
   if (P.n > kRRMaxRows || P.nnz >= (1 << (31 - kTrsvShift))) return;
+  build_compact_programs(P);
+  const int p = P.opts.precond;
+  if (p != BILU_PRECOND_ILU0 && p != BILU_PRECOND_ILU0_SPLIT && p != BILU_PRECOND_PARILU0) return;
+  if (P.tc_mc && (P.n > 1024 || P.opts.reduction != BILU_REDUCE_FAST)) return;
   bilu::build_trsv_program(P.rp.data(), P.ci.data(), P.diag.data(), P.lev_lo_ptr, P.lev_lo_rows, false, P.tp_lo_hdr,
                            P.tp_lo);
   bilu::build_trsv_program(P.rp.data(), P.ci.data(), P.diag.data(), P.lev_up_ptr, P.lev_up_rows, true, P.tp_up_hdr,
                            P.tp_up);
-  build_compact_programs(P);
 }
 
 // SELL-32 layout of a pattern with n <= 1024 rows (DevPattern::sa_* / su_*).
@@ -304,8 +308,10 @@ void build_deps(bilu_plan& P) {
   build_compact_ilu(P);
   P.ilu_hdr.clear();
   P.ilu_prog.clear();
-  // the merged form's in-kernel ILU(0) in the register-resident solver (n <= 1024, 20-bit positions)
-  if (P.n <= 1024 && P.nnz < (1 << 20) && P.opts.precond == BILU_PRECOND_ILU0)
+  // the merged form's in-kernel ILU(0) in the register-resident solver (n <= 1024, 20-bit positions); where there is
+  // a compact program, only the FAST order's occupancy variant reads it
+  if (P.n <= 1024 && P.nnz < (1 << 20) && P.opts.precond == BILU_PRECOND_ILU0 &&
+      (P.ic_hdr.empty() || P.opts.reduction == BILU_REDUCE_FAST))
     bilu::build_ilu_program(P.rp.data(), P.ci.data(), P.diag.data(), P.lev_lo_ptr, P.lev_lo_rows, P.dep_ptr, P.dep,
                             P.opts.ilu_approach, P.ilu_hdr, P.ilu_prog);
 }
@@ -491,7 +497,7 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
   const bool occ_variant = (mask & 16) != 0 && (R == 2 || R == 4 || (R == 8 && pv != 3)) && nt <= occ_nt;
   const bool fp32 = is_fp32(o);
   const int fts = fp32 ? 4 : 8;
-  if (pv == 3 && P.tp_lo.empty()) return false;
+  if (pv == 3 && P.tp_lo.empty() && !P.tc_mc) return false;
   // the merged form factorises in FP64 in the factor slot before rounding to FT
   // more systems than are resident at once; fewer may run on more threads (rr_split) with the same layout
   const int split = rr_split(pv, ref ? 1 : 0, n, nt, 1 << 30, P.nsm);
