@@ -166,15 +166,26 @@ typedef struct bilu_plan_info {
   int operands_in_smem;  /* bit 0: A, bit 1: factors / aiL, bit 2: aiU in shared memory;
                             bit 3: A, and aiU, left in global memory are read from SELL-32
                             copies made by one extra launch each per solve; bit 4: the
-                            occupancy variant of the register-resident kernel */
-  int solver_kernel;     /* 0: one CTA per system, vectors in shared memory (every mode);
-                            1: register-resident (BILU_REDUCE_FAST with n <= 1024, or
-                            ILU factors or none, rows of at most 16 entries and the
-                            reference order with n <= 1024 or either order with
-                            n <= 2048): `threads` threads per system, each owning at
-                            most 8 rows (FAST order with n <= 1024: t + k * threads) */
+                            occupancy variant of the register-resident kernel was asked
+                            for (at 5 to 8 rows per thread the same kernel runs without) */
+  int solver_kernel;     /* 1: register-resident (BILU_REDUCE_FAST with n <= 1024, or
+                            ILU factors or none, rows of at most 16 entries and either
+                            order with n <= 2048): `threads` threads per system, each
+                            owning at most 8 rows (FAST order with n <= 1024:
+                            t + k * threads); with n > 1024, batches of no more systems
+                            than SMs may run on the shared-memory kernel, same bits.
+                            0: every other plan.  threads, smem_bytes and
+                            operands_in_smem then describe the shared-memory kernel;
+                            the reference-order ISAI solvers with n <= 1024 and
+                            threads_per_system 0 run several systems per CTA of their
+                            own (bilu_plan_solver_kernel tells) */
 } bilu_plan_info;
 bilu_status bilu_plan_get_info(const bilu_plan* plan, bilu_plan_info* info);
+/* The solver kernel that bilu_solve runs for a batch of nsys systems (a static
+ * string; NULL for a NULL plan or nsys < 0): k_bicgstab (one CTA per system,
+ * vectors in shared memory), k_bicgstab_isai_ref (several systems per CTA),
+ * k_bicgstab_rr, _rr_lu, _rr_occ, _rr_split, _rr_wide (register-resident). */
+const char* bilu_plan_solver_kernel(const bilu_plan* plan, int nsys);
 
 /* Host copy of a pattern held by the plan.  which: 0 = factor pattern (A with
  * diagonals), 1 = ISAI(L), 2 = ISAI(U), 3 = L (reference L_pages), 4 = U

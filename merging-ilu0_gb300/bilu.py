@@ -28,6 +28,7 @@ REDUCE_REF, REDUCE_FAST = 0, 1
 
 EXPORTED = [
     "bilu_default_options", "bilu_plan_create", "bilu_plan_destroy", "bilu_plan_get_info",
+    "bilu_plan_solver_kernel",
     "bilu_plan_get_pattern", "bilu_expand_values", "bilu_solve", "bilu_solve_warm", "bilu_ilu0",
     "bilu_parilu0", "bilu_split_lu", "bilu_isai", "bilu_true_residual", "bilu_last_error",
     "bilu_version", "bilu_device_count", "bilu_gen_stencil", "bilu_gen_stencil_range", "bilu_gen_uneven",
@@ -92,6 +93,8 @@ def lib():
         L.bilu_plan_create.argtypes = [C.POINTER(vp), i, i, ip, ip, C.POINTER(Options)]
         L.bilu_plan_destroy.argtypes = [vp]
         L.bilu_plan_get_info.argtypes = [vp, C.POINTER(PlanInfo)]
+        L.bilu_plan_solver_kernel.argtypes = [vp, i]
+        L.bilu_plan_solver_kernel.restype = C.c_char_p
         L.bilu_plan_get_pattern.argtypes = [vp, i, ip, ip, ip, ip]
         L.bilu_expand_values.argtypes = [vp, i, vp, vp, vp]
         L.bilu_solve.argtypes = [vp, i, vp, vp, vp, C.POINTER(Results), vp]
@@ -314,6 +317,10 @@ class Plan:
         i = PlanInfo()
         _check(lib().bilu_plan_get_info(self.h, C.byref(i)))
         return {k: getattr(i, k) for k, _ in PlanInfo._fields_}
+
+    def solver_kernel(self, nsys):
+        """Name of the solver kernel that solve() runs for a batch of nsys systems."""
+        return lib().bilu_plan_solver_kernel(self.h, nsys).decode()
 
     def pattern(self, which):
         n, nnz = C.c_int(), C.c_int()

@@ -352,6 +352,8 @@ int rr_slots(int n, int nt);            // the row slots of the kernels: 3 and 6
 int rr_max_threads(int R, bool wide = false);
 int rr_split(int pv, int ref, int n, int nt, int nsys, int nsm);  // threads per order thread of a batch
 const void* rr_kernel(int pv, int fp32, int n, int nt, int ref, int occ, int mc, int split);  // null: no such variant
+// the name of the kernel that launch_solve_rr launches
+const char* rr_kernel_name(int pv, int n, int nt, int ref, int occ, int mc, int nsys, int nsm);
 const void* rr_wide_kernel(int pv, int fp32, int ref, int nt, int mc);      // k_solve_rr_wide.cu
 const void* rr_split_kernel(int pv, int fp32, int split, int slots);        // k_solve_rr_split.cu
 const void* rr_lu_kernel(int fp32, int slots, int ref, int mc);             // k_solve_rr_lu.cu
@@ -455,6 +457,8 @@ struct bilu_plan {
   // register-resident FAST solver (k_solve_rr.cu), when it applies
   bool rr = false;
   int rr_threads = 0, rr_pv = 0;
+  bool isai_ref = false;  // k_bicgstab_isai_ref
+  int isai_maxl = 0;      // longest row of the ISAI patterns
   bool rr_sell = false;  // SpMVs read SELL-32 copies of A (and of aiU) made before the solver launch
   bool rr_occ = false;   // the occupancy variant was asked for (staging bit 4)
   int nsm = 0;           // SMs of the device

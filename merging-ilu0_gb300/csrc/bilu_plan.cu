@@ -591,6 +591,18 @@ void choose_rr(bilu_plan& P) {
   rr_configure(P, nt, o.smem_staging >= 0 ? o.smem_staging : ((split ? 0 : 6) | (lu && P.n > 512 ? 8 : 0)));
 }
 
+// The reference's ISAI solvers: several systems per CTA, unless the caller asked for a CTA size.
+void choose_isai_ref(bilu_plan& P) {
+  const bilu_options& o = P.opts;
+  P.isai_maxl = 0;
+  if (P.has_isai)
+    for (int i = 0; i < P.n; ++i)
+      P.isai_maxl =
+          std::max({P.isai_maxl, P.ail_rp[i + 1] - P.ail_rp[i], P.general_isai ? 0 : P.aiu_rp[i + 1] - P.aiu_rp[i]});
+  P.isai_ref = !P.rr && prec_kind(o.precond) == PK_ISAI && !P.general_isai && o.reduction != BILU_REDUCE_FAST &&
+               o.threads_per_system == 0 && isai_ref_fits(P.n, is_fp32(o) ? 1 : 0, P.a_maxl, P.isai_maxl);
+}
+
 bilu_status upload(bilu_plan& P) {
   std::vector<int> buf;
   auto put = [&](const std::vector<int>& v) {
@@ -1025,6 +1037,7 @@ bilu_status bilu_plan_create(bilu_plan** out, int n, int nnz, const int* h_rp, c
   if (P->has_isai && !P->general_isai) build_sell(n, P->aiu_rp, P->aiu_ci, P->su_off, P->su_ci, P->su_src);
   choose_layout(*P);
   choose_rr(*P);
+  choose_isai_ref(*P);
   if (!P->rr && P->lay.total > (int)solve_max_smem()) {
     const int need = P->lay.total;
     delete P;
@@ -1115,6 +1128,14 @@ bilu_status bilu_plan_autotune(bilu_plan* P, int nsys, const double* d_values, c
   }
   P->timing = had_timing;
   return st;
+}
+
+const char* bilu_plan_solver_kernel(const bilu_plan* P, int nsys) {
+  if (!P || nsys < 0) return nullptr;
+  if (P->isai_ref) return "k_bicgstab_isai_ref";
+  if (!P->rr || takes_shared(*P, nsys)) return "k_bicgstab";
+  return rr_kernel_name(P->rr_pv, P->n, P->rr_threads, P->opts.reduction == BILU_REDUCE_FAST ? 0 : 1, P->rr_occ ? 1 : 0,
+                        P->tc_mc, nsys, P->nsm);
 }
 
 bilu_status bilu_plan_destroy(bilu_plan* P) {
@@ -1298,14 +1319,7 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
       }
     }
   }
-  int maxi = 0;  // longest row of aiL / aiU
-  if (P->has_isai) {
-    for (int i = 0; i < P->n; ++i) {
-      maxi = std::max(maxi, P->ail_rp[i + 1] - P->ail_rp[i]);
-      maxi = std::max(maxi, P->aiu_rp[i + 1] - P->aiu_rp[i]);
-    }
-  }
-  const int maxl = std::max(P->a_maxl, maxi);
+  const int maxl = std::max(P->a_maxl, P->isai_maxl);
   if (P->timing) cudaEventRecord(P->ev[1], st);
   if (sc.sell_u) {
     e = launch_to_sell(P->dp.su_src, P->dp.su_nnz, P->dp.aiu_nnz, nsys, a.aiu, ws + sc.usell, fp32 ? 4 : 8, st);
@@ -1317,12 +1331,9 @@ bilu_status solve_launch(bilu_plan* P, int nsys, const double* vals, const doubl
     if (e != cudaSuccess) return cuda_err(e, "SELL copy of A");
     a.A_sell = (const double*)(ws + sc.asell);
   }
-  // the reference's ISAI solvers: several systems per CTA, unless the caller asked for a CTA size
-  const bool isai_ref = !P->rr && a.prec == PK_ISAI && !P->general_isai && o.reduction != BILU_REDUCE_FAST &&
-                        o.threads_per_system == 0 && isai_ref_fits(P->n, fp32 ? 1 : 0, P->a_maxl, maxi);
   const bool lean = P->rr && rr_takes_lean(*P, nsys);
-  e = isai_ref
-          ? launch_solve_isai_ref(a, fp32 ? 1 : 0, P->a_maxl, maxi, P->nsm, st)
+  e = P->isai_ref
+          ? launch_solve_isai_ref(a, fp32 ? 1 : 0, P->a_maxl, P->isai_maxl, P->nsm, st)
       : P->rr && !takes_shared(*P, nsys)
           ? launch_solve_rr(a, lean ? P->rr_lean : P->rr_lay, P->rr_threads, P->rr_pv, fp32 ? 1 : 0,
                             o.reduction == BILU_REDUCE_FAST ? 0 : lean ? 2 : 1, P->rr_occ ? 1 : 0, P->nsm, st)

@@ -104,6 +104,14 @@ const void* rr_kernel(int pv, int fp32, int n, int nt, int ref, int occ, int mc,
   return fp32 ? rr_kernel_pv<2, float, kFast>(slots) : rr_kernel_pv<2, double, kFast>(slots);
 }
 
+const char* rr_kernel_name(int pv, int n, int nt, int ref, int occ, int mc, int nsys, int nsm) {
+  const int slots = rr_slots(n, nt);
+  if (nt > 128 && slots > 4) return "k_bicgstab_rr_wide";
+  if (rr_split(pv, ref, n, nt, nsys, nsm) > 1) return "k_bicgstab_rr_split";
+  if (occ && slots <= 4) return "k_bicgstab_rr_occ";
+  return pv == 3 && mc ? "k_bicgstab_rr_lu" : "k_bicgstab_rr";
+}
+
 cudaError_t launch_solve_rr(const SolveArgs& a, const RRLayout& L, int nt, int pv, int fp32, int ref, int occ,
                             int nsm, cudaStream_t st) {
   if (a.nsys == 0) return cudaSuccess;
