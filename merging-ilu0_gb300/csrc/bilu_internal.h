@@ -378,7 +378,8 @@ cudaError_t launch_dense_solve(const DevPattern& p, int nsample, const int* sys_
 cudaError_t launch_mlp_rowstats(const DevPattern& p, int nsys, const double* A, float* rown, float* coln, float* corr,
                                 cudaStream_t st);
 size_t mlp_train_smem();
-// loss and gradient of a batch (overwritten); work: mlp_train_work(nrows) bytes for at most nrows blocks at a time
+// loss and gradient of a batch (overwritten); work: mlp_train_work(nrows) bytes for at most 2 nrows blocks at a time,
+// zero before the first call and left as the next one needs it
 int mlp_train_rows(int nsample, int nsm);
 size_t mlp_train_work(int nrows);
 cudaError_t launch_mlp_train(const DevPattern& p, int nsys, const double* A, const double* LUt, const float* rown,

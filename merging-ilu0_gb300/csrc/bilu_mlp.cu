@@ -180,6 +180,7 @@ bilu_status bilu_mlp_train(bilu_mlp* M, const bilu_plan* P, int nsys, const doub
   if (!st) st = ensure_work(M, batch, steps, &nrows, &d_losses);
   if (st) return st;
   cudaError_t e = launch_mlp_rowstats(P->dp, nsys, d_values, rown, coln, corr, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(M->work, 0, mlp_train_work(nrows), s);
   for (int t = 0; t < steps && e == cudaSuccess; ++t) {
     e = launch_mlp_train(P->dp, nsys, d_values, d_lu_target, rown, coln, corr, M->pbf, batch, nullptr,
                          seed ^ (0xA24BAED4963EE407ull * (uint64_t)(M->step + 1)), M->work, nrows, M->g, d_losses + t,
@@ -213,6 +214,7 @@ bilu_status bilu_mlp_loss_grad(bilu_mlp* M, const bilu_plan* P, int nsys, const 
   if (st) return st;
   cudaError_t e = cudaMemcpyAsync(M->idx, h_idx, nsample * sizeof(int), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = launch_mlp_rowstats(P->dp, nsys, d_values, rown, coln, corr, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(M->work, 0, mlp_train_work(nrows), s);
   if (e == cudaSuccess)
     e = launch_mlp_train(P->dp, nsys, d_values, d_lu_target, rown, coln, corr, M->pbf, nsample, M->idx, 0, M->work,
                          nrows, M->g, d_loss, s);

@@ -234,14 +234,19 @@ static_assert(OW2 % 4 == 0 && H * LD * 4 <= TB * TB * 2, "dW2 rows");
 // Layer 1, the activations and the output layer run on the CUDA cores in FP32
 // with the accurate tanh.  Per-unit sums over the block (db1, db2, dW3) are
 // reduce-scattered across each warp; dW1 is reduced over the block in shared
-// memory; the block's share of the gradient and of the loss is row blockIdx.x
-// of `rows` (kTrainRow floats: the gradient, then the loss), which k_grad_sum
-// adds up in a fixed order.  (Atomic additions to one gradient gave other bits
-// on every run: a parameter on a BF16 rounding boundary then moves the losses
-// of the steps that follow, by 1e-7 to 4e-5 over 40 steps.)  Samples: explicit
-// global entry indices (s*nnz+e) or, when idx == NULL, hashed from (seed,
-// sample number).  A tensor-core round that does not complete within the
-// bounded wait leaves a row of zeros with the loss NaN and ends the block.
+// memory; the block's share of the gradient and of the loss is added to row
+// blockIdx.x / 2 of `rows` (kTrainRow floats, zero before: the gradient, then
+// the loss), which k_grad_sum adds up in a fixed order.  Two shares per
+// row, because the sum of zero and two numbers is the same in either order, and
+// half the rows keep a small model's memory within one of the driver's 2 MB
+// chunks (a new one costs 0.17 ms per model: create, 8 steps of 9000 samples
+// and destroy 0.59 ms with a row per block, 0.40 with this).  (Additions of
+// every block to one gradient gave other bits on every run: a parameter on a
+// BF16 rounding boundary then moves the losses of the steps that follow, by
+// 1e-7 to 5e-4 over 40 steps.)  Samples: explicit global entry indices
+// (s*nnz+e) or, when idx == NULL, hashed from (seed, sample number).  A
+// tensor-core round that does not complete within the bounded wait adds NaN to
+// the loss and ends the block.
 __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, const double* __restrict__ A,
                                                   const double* __restrict__ LUt, const float* __restrict__ rown,
                                                   const float* __restrict__ coln, const float* __restrict__ corr,
@@ -293,7 +298,7 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
   // ---- sample, features, target
   const long long q = first + (long long)blockIdx.x * TB + t;
   const bool live = q < nsample;
-  float* grad = rows + (size_t)blockIdx.x * kTrainRow;
+  float* grad = rows + (size_t)(blockIdx.x >> 1) * kTrainRow;
   float f[NF];
   float ytrue = 0.0f;
   if (live) {
@@ -499,9 +504,9 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
         dw2([&](int o, const float(&d3)[16], const float(&d4)[16]) {
 #pragma unroll
           for (int k = 0; k < 16; k += 4)
-            *reinterpret_cast<float4*>(grad + OW2 + t * H + o + k) =
-                make_float4((d3[k] + d4[k]) + W2L[o + k], (d3[k + 1] + d4[k + 1]) + W2L[o + k + 1],
-                            (d3[k + 2] + d4[k + 2]) + W2L[o + k + 2], (d3[k + 3] + d4[k + 3]) + W2L[o + k + 3]);
+            atomicAdd(reinterpret_cast<float4*>(grad + OW2 + t * H + o + k),
+                      make_float4((d3[k] + d4[k]) + W2L[o + k], (d3[k + 1] + d4[k + 1]) + W2L[o + k + 1],
+                                  (d3[k + 2] + d4[k + 2]) + W2L[o + k + 2], (d3[k + 3] + d4[k + 3]) + W2L[o + k + 3]));
         });
       if (t == 0) {
         float a = 0.0f, d = 0.0f;
@@ -509,8 +514,8 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
           a += s_loss[w];
           d += s_do[w];
         }
-        grad[kMlpParams] = a * scale;
-        grad[OB3] = d;
+        atomicAdd(grad + kMlpParams, a * scale);
+        atomicAdd(grad + OB3, d);
       }
       if (t < H) {
         float db2 = 0.0f, dw3 = 0.0f, db1 = 0.0f;
@@ -519,20 +524,19 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
           dw3 += RED[(1 * 4 + w) * H + t];
           db1 += RED[(2 * 4 + w) * H + t];
         }
-        grad[OB2 + t] = db2;
-        grad[OW3 + t] = dw3;
-        grad[OB1 + t] = db1;
+        atomicAdd(grad + OB2 + t, db2);
+        atomicAdd(grad + OW3 + t, dw3);
+        atomicAdd(grad + OB1 + t, db1);
       }
       for (int k = t; k < H * NF; k += TB) {  // dW1[u][f] = sum_t dpre1[t][u] * x[t][f]
         const int u = k / NF, fi = k % NF;
         float acc = 0.0f;
         for (int r = 0; r < TB; ++r) acc = fmaf(G1[r * LD + u], X[r * NF + fi], acc);
-        grad[OW1 + k] = acc;
+        atomicAdd(grad + OW1 + k, acc);
       }
     }
   }
-  if (s_fail)
-    for (int k = t; k < kTrainRow; k += TB) grad[k] = k == kMlpParams ? __int_as_float(0x7fc00000) : 0.0f;
+  if (s_fail && t == 0) atomicAdd(grad + kMlpParams, __int_as_float(0x7fc00000));
   // a round that timed out may still be in flight: wait once more (bounded) before freeing its columns
   if (s_fail) tc::mbar_wait(&s_mbar, (uint32_t)(s_fail - 1), kWaitLimit);
   tc::fence_before_sync();
@@ -548,22 +552,31 @@ __global__ void __launch_bounds__(TB) k_mlp_train(const DevPattern P, int nsys, 
 // correctly rounded value but for a few ulps of the errors' own sum: nearer to
 // it than any order of plain additions.  acc / cor: the sum and its error so
 // far, continued over the parts of a large batch (start: its first part).
-// Reads 19.5 KB per row: 512 rows (65536 samples) about 4 us.
+// Leaves the rows zero for the next part.
+// Reads 19.5 KB per row: 256 rows (65536 samples) about 3 us.
 constexpr int kSumWarps = 16;
 __device__ __forceinline__ void two_sum(float& s, float& c, float x) {
   const float t = s + x, z = t - s;
   c += (s - (t - z)) + (x - z);
   s = t;
 }
-__global__ void __launch_bounds__(32 * kSumWarps) k_grad_sum(const float* __restrict__ rows, int nrows, int start,
+__global__ void __launch_bounds__(32 * kSumWarps) k_grad_sum(float* rows, int nrows, int start,
                                                             float* __restrict__ acc, float* __restrict__ cor,
                                                             float* __restrict__ grad, float* __restrict__ loss) {
   __shared__ float s_s[kSumWarps][32], s_c[kSumWarps][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
   float s = 0.0f, c = 0.0f;
   if (k <= kMlpParams) {
-#pragma unroll 8
-    for (int r = warp; r < nrows; r += kSumWarps) two_sum(s, c, __ldg(rows + (size_t)r * kTrainRow + k));
+    for (int r = warp; r < nrows; r += 8 * kSumWarps) {
+      float x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = r + j * kSumWarps < nrows ? rows[(size_t)(r + j * kSumWarps) * kTrainRow + k] : 0.0f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        two_sum(s, c, x[j]);
+        if (r + j * kSumWarps < nrows) rows[(size_t)(r + j * kSumWarps) * kTrainRow + k] = 0.0f;
+      }
+    }
   }
   s_s[warp][lane] = s;
   s_c[warp][lane] = c;
@@ -906,18 +919,20 @@ cudaError_t launch_mlp_train(const DevPattern& p, int nsys, const double* A, con
   if (e != cudaSuccess) return e;
   float *acc = work, *cor = work + kTrainRow, *rows = work + 2 * kTrainRow;
   const long long blocks = ((long long)nsample + TB - 1) / TB;
-  for (long long b = 0; b < blocks; b += nrows) {
-    const int part = (int)std::min<long long>(nrows, blocks - b);
+  for (long long b = 0; b < blocks; b += 2LL * nrows) {
+    const int part = (int)std::min<long long>(2LL * nrows, blocks - b), used = (part + 1) / 2;
     k_mlp_train<<<part, TB, smem, st>>>(p, nsys, A, LUt, rown, coln, corr, (const __nv_bfloat16*)pbf, nsample, idx,
                                         seed, 1.0f / (float)nsample, b * TB, rows);
-    k_grad_sum<<<(kMlpParams + 32) / 32, 32 * kSumWarps, 0, st>>>(rows, part, b == 0, acc, cor, grad, loss);
+    k_grad_sum<<<(kMlpParams + 32) / 32, 32 * kSumWarps, 0, st>>>(rows, used, b == 0, acc, cor, grad, loss);
   }
   return cudaGetLastError();
 }
 
-// Rows of the gradient parts kept at a time: one per block, at most eight per SM (24 MB), whole waves of the
+// Rows of the gradient parts kept at a time: one per two blocks, at most four per SM (12 MB), whole waves of the
 // training kernel's one CTA per SM.
-int mlp_train_rows(int nsample, int nsm) { return (int)std::min(((long long)nsample + TB - 1) / TB, 8LL * nsm); }
+int mlp_train_rows(int nsample, int nsm) {
+  return (int)std::min(((long long)nsample + 2 * TB - 1) / (2 * TB), 4LL * nsm);
+}
 size_t mlp_train_work(int nrows) { return (size_t)(nrows + 2) * kTrainRow * sizeof(float); }
 
 cudaError_t launch_mlp_adam(float* p, float* m, float* v, const float* g, void* pbf, int count, float lr, int step,
