@@ -113,9 +113,8 @@ typedef struct bilu_options {
                                 Bit 4: the kernel variant bounded for occupancy (same
                                 arithmetic, fewer registers, more threads per SM): 3 or 4
                                 rows per thread on 4 CTAs of 256 (3 with ILU factors), 2
-                                rows on 2 CTAs of 512; ignored for ILU factors at 5 to 8
-                                rows per thread; without them those rows always run on
-                                two or four threads per system thread, same arithmetic.   */
+                                rows on 2 CTAs of 512; at 5 to 8 rows per thread the same
+                                kernels run with it and without.                          */
 } bilu_options;
 
 /* Fills *opts with the reference defaults: merged ILU(0), approach 1, 5 sweeps,

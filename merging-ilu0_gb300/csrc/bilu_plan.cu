@@ -467,10 +467,10 @@ void choose_layout(bilu_plan& P) {
 // operands that would cost occupancy are left in global memory, read through
 // L1; ILU factors are always staged; bit 3: the SpMVs read SELL-32 copies of
 // the operands left in global memory; bit 4: the occupancy variant of the
-// kernel (k_bicgstab_rr_occ: 4 rows on 4 CTAs of 256 (3 with ILU factors), 2
-// rows on 2 CTAs of 512; ignored for ILU factors at 5 to 8 rows per thread, and
-// without them those have just one kernel, k_bicgstab_rr_split); false when the kernel does not apply or
-// that configuration is invalid.
+// kernel (k_bicgstab_rr_occ: 3 or 4 rows on 4 CTAs of 256 (3 with ILU factors),
+// 2 rows on 2 CTAs of 512; at 5 to 8 rows without ILU factors it is accepted and
+// the kernels are the same, with them it is ignored)); false when the kernel
+// does not apply or that configuration is invalid.
 bool rr_configure(bilu_plan& P, int nt, int mask) {
   const bilu_options& o = P.opts;
   const int pk = prec_kind(o.precond);
@@ -491,8 +491,7 @@ bool rr_configure(bilu_plan& P, int nt, int mask) {
     if ((pv != 0 && pv != 3) || P.a_maxl > 16) return false;
     mask &= 7;
   }
-  // bit 4: the occupancy variant, for 2, 4 or 8 rows per thread (ILU factors: 2 or 4) and at most its
-  // launch bound of threads
+  // bit 4, reported as asked for: at 8 rows rr_kernel has no occupancy variant to choose
   const int occ_nt = R == 8 ? 128 : (R == 4 ? 256 : 512);
   const bool occ_variant = (mask & 16) != 0 && (R == 2 || R == 4 || (R == 8 && pv != 3)) && nt <= occ_nt;
   const bool fp32 = is_fp32(o);

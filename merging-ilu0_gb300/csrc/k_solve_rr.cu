@@ -8,8 +8,8 @@ namespace bilu {
 namespace {
 
 // one CTA per system of a batch sharing one pattern
-// REF: the reference's operation order.  Warp w's lane l owns rows
-// l + 32 (w R + k), a block of the reference's lane-strided inner-product
+// ORD = kRef, kRefLean: the reference's operation order.  Warp w's lane l owns
+// rows l + 32 (w R + k), a block of the reference's lane-strided inner-product
 // terms; the inner products chain through the warps in order (ref_chain_sum),
 // so every scalar is the reference's bit for bit.
 template <int R, int PV, typename FT, int ORD>

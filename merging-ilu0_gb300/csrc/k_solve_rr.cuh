@@ -25,17 +25,21 @@
 // 200 KB CTA per SM, warp-0 inner products (32 dependent FMAs at n = 1000) and
 // ~15 block barriers per iteration during which the SM's FP64 pipes idle.
 // Here:
-//   * thread t of an NT-thread CTA owns rows t + k*NT, k < R (R <= 8); the
-//     vectors x, r/s, p, v and t live in its registers (r_hat = b is re-read
-//     through L1, p_hat / s_hat are read back from shared memory);
+//   * thread t of an NT-thread CTA owns rows t + k*NT, k < R (R <= 8; two or
+//     four threads a part of an order thread's rows each where SPLIT > 1, a
+//     block of 32 R rows per warp in the reference's order); the vectors x,
+//     r/s, p, v and t live in its registers (r_hat = b is re-read through L1,
+//     p_hat / s_hat are read back from shared memory);
 //   * shared memory holds only what other rows read: the SpMV input p_hat /
 //     s_hat (FP64), the preconditioner input and intermediate (FT), and, when
 //     they fit without costing occupancy, A and the ISAI values;
 //   * the six inner products of an iteration run as four block reductions
-//     in one shared slot (orders below); warp 0 alone forms the scalar
-//     recurrence (divisions, square roots, the next beta) and broadcasts it
-//     through shared memory, so those FP64 instructions run once per CTA, not
-//     once per warp; 13 barriers per iteration besides the preconditioner's;
+//     in one shared slot (orders below); one warp alone (warp 0; where sums
+//     chain through the warps the last one, or the last part's first) forms
+//     the scalar recurrence (divisions, square roots, the next beta) and
+//     broadcasts it through shared memory, so those FP64 instructions run once
+//     per CTA, not once per warp; 13 barriers per iteration besides the
+//     preconditioner's (a split or chained sum adds one per part);
 //   * the CTA is small (one warp for n <= 256), so several systems share an SM
 //     and one system's barrier or reduction latency overlaps another's FMAs;
 //   * with FP32 ISAI values (BILU_FP32) both preconditioner SpMVs run on the
@@ -294,9 +298,9 @@ enum RROrder : int { kFast = 0, kRef = 1, kRefLean = 2, kFastChain = 3 };
 
 // Barrier at the end of a level.  WIDE: of the solve's `team` threads, one
 // warp per 32 rows of the widest level (a warp barrier for one warp); the other
-// warps wait once, at the end of the apply.  Otherwise of the CTA: with one
-// CTA of at most four warps per system, a choice of the team in these kernels
-// costs more than the idle warps do (a second copy of the solves: 3D
+// warps wait once, at the end of the apply.  Otherwise of the CTA: at the
+// default of at most four warps per system, a choice of the team in these
+// kernels costs more than the idle warps do (a second copy of the solves: 3D
 // 10x10x10 6.26 -> 6.66 ms, uneven batches 3.33 -> 3.69 ms; a branch per
 // level: 6.53 and 3.45 ms).
 template <bool WIDE>
@@ -339,7 +343,9 @@ __device__ __forceinline__ void tri_solve(const int2* __restrict__ hdr, const in
   // most two entries (5-point stencils) run a copy of the row code with two
   // product slots instead of kTrsvPrefetch: a guarded FMA can be if-converted
   // into a predicated one, which still takes its FP64-unit slot on GB300.
-  // Measured (CUDA events): 2D 16x16 reference order 1.01 -> 1.12M systems/s,
+  // (Grids run the compact programs now; the copy serves the occupancy variant
+  // and schedules past their slot limit.)
+  // Measured before those (CUDA events): 2D 16x16 reference order 1.01 -> 1.12M systems/s,
   // FAST with the reference's stopping rule 84.2 -> 68.7 ms, 24x24 414k ->
   // 423k; 3D 10x10x10 (three entries per row) unchanged.  The choice is one
   // uniform branch between two fully unrolled copies (a per-slot runtime bound
